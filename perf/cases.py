@@ -38,21 +38,21 @@ TYPES = {"bf16": torch.bfloat16, "f16": torch.float16}
 def listed():
     return [
         # one person at a chat window; a server under load; the default type of the served project
-        dict(name="decode, 1 sequence", kind="decode", dtype="bf16", batch=1, ctx=700),
-        dict(name="decode, 64 sequences", kind="decode", dtype="bf16", batch=64, ctx=900),
-        dict(name="decode, 16 sequences, f16", kind="decode", dtype="f16", batch=16, ctx=100),
+        dict(name="decode 1 sequence", kind="decode", dtype="bf16", batch=1, ctx=700),
+        dict(name="decode 64 sequences", kind="decode", dtype="bf16", batch=64, ctx=900),
+        dict(name="decode 16 sequences in f16", kind="decode", dtype="f16", batch=16, ctx=100),
         # a document to read; a draft of eight tokens to check; a scheduler's step with newcomers in it
-        dict(name="prefill, 2000 tokens", kind="prefill", dtype="bf16", tokens=2000),
-        dict(name="verify, 8 tokens", kind="verify", dtype="bf16", tokens=8, ctx=1500),
+        dict(name="prefill 2000 tokens", kind="prefill", dtype="bf16", tokens=2000),
+        dict(name="verify 8 tokens", kind="verify", dtype="bf16", tokens=8, ctx=1500),
         dict(name="mixed step", kind="mixed", dtype="bf16", batch=40, ctx=600, prompts=3, tokens=437),
-        dict(name="serve, Latarax", kind="serve", dtype="bf16", batch=12, tokens=250, steps=6),
+        dict(name="serve Latarax", kind="serve", dtype="bf16", batch=12, tokens=250, steps=6),
         # sampling at the vocabulary of the flagship model; a long context; a product with a ragged batch
-        dict(name="sample, 64 rows", kind="sample", rows=64, vocab=128256, top_p=0.9, penalties=False),
-        dict(name="attention, long contexts", kind="attention", dtype="bf16", batch=20, heads=32, kv=8, ctx=9000, splits=1, window=0),
-        dict(name="gemm, 1500 rows", kind="gemm", dtype="bf16", rows=1500, n=14336, k=4096),
-        dict(name="experts, 600 rows", kind="experts", rows=600, experts=8, top=2, width=4096, ff=7168),
+        dict(name="sample 64 rows", kind="sample", rows=64, vocab=128256, top_p=0.9, penalties=False),
+        dict(name="attention long contexts", kind="attention", dtype="bf16", batch=20, heads=32, kv=8, ctx=9000, splits=1, window=0),
+        dict(name="gemm 1500 rows", kind="gemm", dtype="bf16", rows=1500, n=14336, k=4096),
+        dict(name="experts 600 rows", kind="experts", rows=600, experts=8, top=2, width=4096, ff=7168),
         # the smallest calls: between the products of one layer for one token
-        dict(name="glue, 1 token", kind="glue", dtype="f16", tokens=1),
+        dict(name="glue 1 token", kind="glue", dtype="f16", tokens=1),
     ]
 
 
