@@ -245,6 +245,23 @@ def test_gemm_bf16_tensor_core(hb, cuda, M, N, K_):
     assert rel_err(host(y), K.round_bf16(want)) <= 4e-3
 
 
+@pytest.mark.parametrize("M,N,K_", [(1, 8, 8), (1, 4096, 4096), (17, 136, 72), (64, 4096, 1024), (128, 6144, 512),
+                                    (130, 264, 520), (3, 12, 64), (40, 1000, 4104)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gemm_f16(hb, cuda, M, N, K_, shift):
+    """f16 rows of 16-byte multiples run on the tensor cores; operands one element off a 16-byte boundary (shift) and
+    other widths on the CUDA cores.  Bound: the f16 rounding of the result and K fp32 additions."""
+    g = torch.Generator().manual_seed(M + N + K_)
+    x = torch.empty(M * K_ + 8, dtype=torch.float16, device=cuda)[shift:shift + M * K_].view(M, K_)
+    x.copy_(torch.randn(M, K_, generator=g))
+    w = (torch.randn(N, K_, generator=g) * 0.02).to(cuda, torch.float16)
+    y = hb.gemm(x, w)
+    torch.cuda.synchronize()
+    want = x.double() @ w.double().T
+    bound = want.abs() * 2.0 ** -11 + (x.double().abs() @ w.double().abs().T) * K_ * 2.0 ** -24 + 2.0 ** -25
+    assert bool(((y.double() - want).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
 @pytest.mark.parametrize("M,N,K_", [(1, 32000, 256), (8, 688, 256), (5, 256, 688), (3, 7, 5)])
 def test_gemm_simt_shapes(hb, cuda, dtype, M, N, K_):

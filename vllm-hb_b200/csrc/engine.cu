@@ -198,7 +198,7 @@ static int setup_shape(hb_engine* e, const hb_model_shape& s) {
   e->qkv_rows = (e->hq_l + 2 * e->hkv_l) * e->hd;
   const char* g = getenv("HB_GEMM");
   const bool want_simt = g && std::string(g) == "simt";
-  e->use_tc = !want_simt && e->dtype == HB_BF16 && e->H % 64 == 0 && (e->hq_l * e->hd) % 64 == 0 &&
+  e->use_tc = !want_simt && e->dtype != HB_F32 && e->H % 64 == 0 && (e->hq_l * e->hd) % 64 == 0 &&
               e->I_l % 64 == 0;
   // expert boundaries must fall on 128-feature tiles of the SwiGLU GEMM
   if (e->moe && e->I_l % 128 != 0) e->use_tc = false;
@@ -377,12 +377,14 @@ static int ensure_plans(hb_engine* e, int B, bool chunk, StepPlans** out) {
     // Single rank: residual add and RMSNorm ride in the GEMM epilogues (HB_DEFER_NORM=0:
     // separate add+norm kernels) when o_proj and down_proj get cluster plans.
     static const bool no_defer = [] { const char* v = getenv("HB_DEFER_NORM"); return v && v[0] == '0'; }();
-    sp.defer_norm = e->ws == 1 && !no_defer && e->H % 128 == 0 && !e->moe;  // the router reads normalised x
+    // (the router reads normalised x; and in f16 h * norm_w, which no row scale has brought near one,
+    // can leave the type's range or reach its subnormals)
+    sp.defer_norm = e->ws == 1 && !no_defer && e->H % 128 == 0 && !e->moe && e->dtype == HB_BF16;
     if (sp.defer_norm) {
       TcGemmPlan probe_o, probe_d;
       auto& w0 = e->layers[0];
-      if ((rc = gemm_tc_plan(&probe_o, e->d_attn, w0.wo, B, e->H, e->hq_l * e->hd, kEpiResidual, false, e->device))) return rc;
-      if ((rc = gemm_tc_plan(&probe_d, e->d_act, w0.wdown, B, e->H, e->I_e, kEpiResidual, false, e->device))) return rc;
+      if ((rc = gemm_tc_plan(&probe_o, e->d_attn, w0.wo, B, e->H, e->hq_l * e->hd, kEpiResidual, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
+      if ((rc = gemm_tc_plan(&probe_d, e->d_act, w0.wdown, B, e->H, e->I_e, kEpiResidual, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
       sp.defer_norm = probe_o.cluster && probe_d.cluster && probe_o.m_tiles == 1 && probe_d.m_tiles == 1;
     }
     // Several ranks: the row-parallel GEMMs push their partial tiles straight into the
@@ -400,8 +402,8 @@ static int ensure_plans(hb_engine* e, int B, bool chunk, StepPlans** out) {
       if (sp.push) {
         TcGemmPlan probe_o, probe_d;
         auto& w0 = e->layers[0];
-        if ((rc = gemm_tc_plan(&probe_o, e->d_attn, w0.wo, B, e->H, e->hq_l * e->hd, kEpiPush, false, e->device))) return rc;
-        if ((rc = gemm_tc_plan(&probe_d, e->d_act, w0.wdown, B, e->H, e->I_e, kEpiPush, false, e->device))) return rc;
+        if ((rc = gemm_tc_plan(&probe_o, e->d_attn, w0.wo, B, e->H, e->hq_l * e->hd, kEpiPush, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
+        if ((rc = gemm_tc_plan(&probe_d, e->d_act, w0.wdown, B, e->H, e->I_e, kEpiPush, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
         const int tiles = (int)(e->H / 128 / e->ws);
         sp.geo_o = {gemm_tc_push_row_block(probe_o), tiles};
         sp.geo_down = {gemm_tc_push_row_block(probe_d), tiles};
@@ -411,23 +413,23 @@ static int ensure_plans(hb_engine* e, int B, bool chunk, StepPlans** out) {
     const int row_epi = sp.defer_norm ? kEpiResidual : (sp.push ? kEpiPush : kEpiStore);
     for (int64_t l = 0; l < e->L; ++l) {
       auto& w = e->layers[l];
-      if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kQkv], e->d_x, w.wqkv, B, e->qkv_rows, e->H, kEpiStore, false, e->device))) return rc;
-      if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kO], e->d_attn, w.wo, B, e->H, e->hq_l * e->hd, row_epi, false, e->device))) return rc;
+      if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kQkv], e->d_x, w.wqkv, B, e->qkv_rows, e->H, kEpiStore, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
+      if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kO], e->d_attn, w.wo, B, e->H, e->hq_l * e->hd, row_epi, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
       if (e->fused_swiglu) {
-        if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kGateUp], e->d_x, w.wgu, B, 2 * e->I_e, e->H, kEpiSwiGLU, false, e->device))) return rc;
+        if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kGateUp], e->d_x, w.wgu, B, 2 * e->I_e, e->H, kEpiSwiGLU, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
       } else {
-        if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kGateUp], e->d_x, w.wgu, B, 2 * e->I_e, e->H, kEpiStore, false, e->device))) return rc;
+        if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kGateUp], e->d_x, w.wgu, B, 2 * e->I_e, e->H, kEpiStore, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
       }
-      if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kDown], e->d_act, w.wdown, B, e->H, e->I_e, row_epi, false, e->device))) return rc;
+      if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kDown], e->d_act, w.wdown, B, e->H, e->I_e, row_epi, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
       for (int k = 0; k < 4; ++k) ws = std::max(ws, sp.layer[l * 4 + k].workspace_bytes());
     }
-    if ((rc = gemm_tc_plan(&sp.lm_head, e->d_x, e->lm_head, B, e->V, e->H, kEpiStore, true, e->device))) return rc;
+    if ((rc = gemm_tc_plan(&sp.lm_head, e->d_x, e->lm_head, B, e->V, e->H, kEpiStore, true, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
     ws = std::max(ws, sp.lm_head.workspace_bytes());
     // RoPE and the KV write ride in the q|k|v GEMM epilogue when its output tile is one head
     // (HB_ROPE_EPI=0: the separate kernel)
     const char* re_env = getenv("HB_ROPE_EPI");  // read per plan, so that tests can compare both forms
     const bool no_rope_epi = re_env && re_env[0] == '0';
-    sp.rope_epi = !no_rope_epi && e->dtype == HB_BF16 && e->hd == 128 && e->L > 0 &&
+    sp.rope_epi = !no_rope_epi && e->hd == 128 && e->L > 0 &&
                   gemm_tc_rope_epilogue_ok(sp.layer[kQkv]);
     if (sp.defer_norm) {
       auto can_scale = [](const TcGemmPlan& pl) { return pl.tma_store && (pl.cluster || pl.splits == 1) && pl.m_tiles == 1; };
@@ -438,8 +440,8 @@ static int ensure_plans(hb_engine* e, int B, bool chunk, StepPlans** out) {
         sp.defer_norm = false;
         for (int64_t l = 0; l < e->L; ++l) {
           auto& w = e->layers[l];
-          if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kO], e->d_attn, w.wo, B, e->H, e->hq_l * e->hd, kEpiStore, false, e->device))) return rc;
-          if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kDown], e->d_act, w.wdown, B, e->H, e->I_e, kEpiStore, false, e->device))) return rc;
+          if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kO], e->d_attn, w.wo, B, e->H, e->hq_l * e->hd, kEpiStore, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
+          if ((rc = gemm_tc_plan(&sp.layer[l * 4 + kDown], e->d_act, w.wdown, B, e->H, e->I_e, kEpiStore, false, e->device, 0, nullptr, nullptr, e->dtype))) return rc;
         }
       }
     }

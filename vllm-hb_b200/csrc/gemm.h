@@ -160,6 +160,7 @@ struct TcGemmPlan {
   GatedAct act2;
   int64_t ldx = 0, ldy = 0;
   bool out_f32 = false;
+  hb_dtype dtype = HB_BF16;  // of X, W and 16-bit outputs
   bool tma_store = false;  // output rows are 16-byte multiples: bulk tensor stores
   // scratch layout inside the caller's workspace
   size_t ws_partials_bytes = 0;  // fp32 [m_tiles*n_tiles*splits][m_pad][128]
@@ -171,7 +172,7 @@ bool gemm_tc_supported(int64_t M, int64_t N, int64_t K, hb_dtype dtype);
 // X and W must be 16-byte aligned device pointers; they are baked into the plan.
 int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int64_t N, int64_t K,
                  int epilogue, bool out_f32, int device, int force_splits = 0, const TcGroups* groups = nullptr,
-                 const TcHeads* heads = nullptr);
+                 const TcHeads* heads = nullptr, hb_dtype dtype = HB_BF16);
 // groups: W holds the [N, K] matrices of all groups one after another, M is the row capacity of the
 // sorted batch operand; gemm_tc_run then needs tile_group (device, max_tiles entries).
 // Y row stride ldy in elements.  workspace: plan.workspace_bytes(), zeroed once.

@@ -1,4 +1,4 @@
-// bf16 GEMM for decode shapes on 5th-generation tensor cores (tcgen05 + TMEM + TMA).
+// bf16 and f16 GEMM for decode shapes on 5th-generation tensor cores (tcgen05 + TMEM + TMA).
 //
 //   Y[M,N] = X[M,K] . W[N,K]^T        M = batch (1..256 per tile), weights [out,in]
 //
@@ -63,7 +63,7 @@ struct TcParams {
   // row sums of h^2 over this tile's 128 features to rowsq_out[row * rowsq_stride + tile].
   // Consumer (rowsq_in != null): every accumulator column (batch row) is multiplied by
   // rsqrt(sum over rowsq_tiles entries / rs_n + rs_eps) before the epilogue.
-  const __nv_bfloat16* norm_w;
+  const void* norm_w;
   float* rowsq_out;
   const float* rowsq_in;
   int rowsq_stride, rowsq_tiles;
@@ -75,8 +75,8 @@ struct TcParams {
   // RoPE + paged KV write (see TcNormLink): tile t is head t of the [q|k|v] row.
   const float2* rope_cs;
   const int64_t* kv_slots;
-  __nv_bfloat16* k_cache;
-  __nv_bfloat16* v_cache;
+  void* k_cache;
+  void* v_cache;
   int rope_nq, rope_nkv;
   int64_t kv_num_blocks;
   // kEpiPush (see TcNormLink): staging bases of all ranks, this rank, tiles and 16-byte
@@ -212,7 +212,8 @@ __device__ __forceinline__ float gated_f(float g, float u, const GatedAct& act) 
 // HEADS: blockIdx.z counts independent products (TcHeads).  The instance without any of them is the
 // one decode steps of dense models run: whatever it does not need costs it registers and time (2 % of
 // an 8B step).
-template <bool GROUPS, bool GENERAL, bool HEADS>
+// T: type of the operands and of 16-bit outputs (bf16 or f16).
+template <bool GROUPS, bool GENERAL, bool HEADS, typename T = __nv_bfloat16>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_h,
@@ -424,7 +425,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   } else if (warp == 1) {
     if (lane == 0) {
       // ------------------------------------------------------------ MMA issuer
-      const uint32_t idesc = make_idesc(p.m_pad);
+      const uint32_t idesc = make_idesc<T>(p.m_pad);
       bool ok = true;
       for (int i = 0; i < n_kc && ok; ++i) {
         const int s = i % p.stages;
@@ -557,7 +558,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const bool ok_recv = ok_all && mbar_wait(smem_u32(&s_recv), 0, &s_abort);
     TC_TRACE(tid == 0, 6);
     bool resid_ok = true;
-    const float w_norm = (residual && n_glob < p.N) ? __bfloat162float(p.norm_w[n_glob]) : 0.f;
+    const float w_norm = (residual && n_glob < p.N) ? to_f32<T>(((const T*)p.norm_w)[n_glob]) : 0.f;
     if (ok_recv) {
       const int c_lo = split * CW;
       for (int c0 = c_lo & ~15; c0 < c_lo + CW; c0 += 16) {
@@ -619,17 +620,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             const bool landed = mbar_wait(smem_u32(&s_resid), 0, &s_abort);
             resid_ok = resid_ok && landed;
           }
-          const __nv_bfloat16* rs_tile = reinterpret_cast<const __nv_bfloat16*>(smem_gen + resid_off);
-          __nv_bfloat16* hs = reinterpret_cast<__nv_bfloat16*>(smem_gen + h_off);
-          __nv_bfloat16* ts = reinterpret_cast<__nv_bfloat16*>(smem_gen + out_off);
+          const T* rs_tile = reinterpret_cast<const T*>(smem_gen + resid_off);
+          T* hs = reinterpret_cast<T*>(smem_gen + h_off);
+          T* ts = reinterpret_cast<T*>(smem_gen + out_off);
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int cl = c0 + j - c_lo;
             if (cl >= 0 && cl < CW) {
-              const float y = __bfloat162float(__float2bfloat16_rn(g[j]));
-              const __nv_bfloat16 h = __float2bfloat16_rn(__bfloat162float(rs_tile[cl * kTileN + row]) + y);
+              const float y = to_f32<T>(from_f32<T>(g[j]));
+              const T h = from_f32<T>(to_f32<T>(rs_tile[cl * kTileN + row]) + y);
               hs[cl * kTileN + row] = h;
-              ts[cl * kTileN + row] = __float2bfloat16_rn(__bfloat162float(h) * w_norm);
+              ts[cl * kTileN + row] = from_f32<T>(to_f32<T>(h) * w_norm);
             }
           }
         } else {
@@ -638,7 +639,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             const int cl = c0 + j - c_lo;
             if (cl >= 0 && cl < CW) {
               if (p.out_f32) reinterpret_cast<float*>(smem_gen + out_off)[cl * kTileN + row] = g[j];
-              else reinterpret_cast<__nv_bfloat16*>(smem_gen + out_off)[cl * kTileN + row] = __float2bfloat16_rn(g[j]);
+              else reinterpret_cast<T*>(smem_gen + out_off)[cl * kTileN + row] = from_f32<T>(g[j]);
             }
           }
         }
@@ -651,12 +652,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     if (tail_ok && residual) {
       // sum of squares of every new residual row over this tile's 128 features: a warp per
       // row, four values per lane, fixed order
-      const __nv_bfloat16* hs = reinterpret_cast<const __nv_bfloat16*>(smem_gen + h_off);
+      const T* hs = reinterpret_cast<const T*>(smem_gen + h_off);
       for (int cl = warp; cl < CW; cl += kTcThreads / 32) {
         const uint2 raw = *reinterpret_cast<const uint2*>(hs + cl * kTileN + lane * 4);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-        const float2 a = __bfloat1622float2(h2[0]), b = __bfloat1622float2(h2[1]);
-        float ss = (a.x * a.x + a.y * a.y) + (b.x * b.x + b.y * b.y);
+        const T* h4 = reinterpret_cast<const T*>(&raw);
+        const float a0 = to_f32<T>(h4[0]), a1 = to_f32<T>(h4[1]), b0 = to_f32<T>(h4[2]), b1 = to_f32<T>(h4[3]);
+        float ss = (a0 * a0 + a1 * a1) + (b0 * b0 + b1 * b1);
         ss = warp_sum(ss);
         const int m = m_base + split * CW + cl;
         if (lane == 0 && m < p.M) p.rowsq_out[(int64_t)m * p.rowsq_stride + tile] = ss;
@@ -667,18 +668,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       // the staged tile is one head for this CTA's CW batch rows: rotate query and key heads
       // (pairs (i, i + 64), values as rounded to bf16 above), send key and value heads
       // straight to their cache slots
-      __nv_bfloat16* ts = reinterpret_cast<__nv_bfloat16*>(smem_gen + out_off);
+      T* ts = reinterpret_cast<T*>(smem_gen + out_off);
       const int head = tile, row0 = m_base + split * CW;
       if (tail_ok && head < p.rope_nq + p.rope_nkv) {
         for (int idx = tid; idx < CW * 64; idx += kTcThreads) {
           const int cl = idx >> 6, i = idx & 63, m = row0 + cl;
           if (m < p.M) {
             const float2 cs = __ldg(p.rope_cs + (int64_t)m * 64 + i);
-            const float x1 = __bfloat162float(ts[cl * kTileN + i]), x2 = __bfloat162float(ts[cl * kTileN + 64 + i]);
+            const float x1 = to_f32<T>(ts[cl * kTileN + i]), x2 = to_f32<T>(ts[cl * kTileN + 64 + i]);
             float o1, o2;
             rope_rotate(x1, x2, cs.x, cs.y, &o1, &o2);
-            ts[cl * kTileN + i] = __float2bfloat16_rn(o1);
-            ts[cl * kTileN + 64 + i] = __float2bfloat16_rn(o2);
+            ts[cl * kTileN + i] = from_f32<T>(o1);
+            ts[cl * kTileN + 64 + i] = from_f32<T>(o2);
           }
         }
       }
@@ -688,7 +689,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         store_y = false;
         if (tail_ok) {
           const bool is_k = head < p.rope_nq + p.rope_nkv;
-          __nv_bfloat16* cache = is_k ? p.k_cache : p.v_cache;
+          T* cache = (T*)(is_k ? p.k_cache : p.v_cache);
           const int kvh = head - p.rope_nq - (is_k ? 0 : p.rope_nkv);
           for (int idx = tid; idx < CW * 16; idx += kTcThreads) {
             const int cl = idx >> 4, v = idx & 15, m = row0 + cl;
@@ -696,7 +697,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
               const int64_t slot = __ldg(p.kv_slots + m);
               if (slot >= 0 && slot < p.kv_num_blocks * HB_BLOCK_SIZE) {
                 const int64_t blk = slot / HB_BLOCK_SIZE, off = slot % HB_BLOCK_SIZE;
-                __nv_bfloat16* dst = cache + ((blk * p.rope_nkv + kvh) * HB_BLOCK_SIZE + off) * (int64_t)kTileN;
+                T* dst = cache + ((blk * p.rope_nkv + kvh) * HB_BLOCK_SIZE + off) * (int64_t)kTileN;
                 reinterpret_cast<uint4*>(dst)[v] = reinterpret_cast<const uint4*>(ts + cl * kTileN)[v];
               }
             }
@@ -766,7 +767,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           if (p.out_f32) reinterpret_cast<float*>(dst)[j * kTileN + row] = v[j];
-          else reinterpret_cast<__nv_bfloat16*>(dst)[j * kTileN + row] = __float2bfloat16_rn(v[j]);
+          else reinterpret_cast<T*>(dst)[j * kTileN + row] = from_f32<T>(v[j]);
         }
       }
       fence_async_smem();
@@ -805,7 +806,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             const int m = m_base + c0 + j;
             if (m < p.M) {
               if (p.out_f32) ((float*)p.Y)[(int64_t)m * p.ldy + n_glob] = v[j];
-              else ((__nv_bfloat16*)p.Y)[(int64_t)m * p.ldy + n_glob] = __float2bfloat16_rn(v[j]);
+              else ((T*)p.Y)[(int64_t)m * p.ldy + n_glob] = from_f32<T>(v[j]);
             }
           }
         }
@@ -857,7 +858,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             if (m < m_lim && n_glob < p.N) {
               const float r = swiglu ? gated(g[j], u[j]) : g[j];
               if (p.out_f32) ((float*)p.Y)[(int64_t)(m_base + m) * p.ldy + n_glob] = r;
-              else ((__nv_bfloat16*)p.Y)[(int64_t)(m_base + m) * p.ldy + n_glob] = __float2bfloat16_rn(r);
+              else ((T*)p.Y)[(int64_t)(m_base + m) * p.ldy + n_glob] = from_f32<T>(r);
             }
           }
         }
@@ -911,37 +912,40 @@ static EncodeTiledFn get_encode() {
   return fn;
 }
 
-// 2-D bf16 row-major [rows, cols] tensor, box [box_rows, 64 cols], 128-byte swizzle.
+static CUtensorMapDataType tm_type(hb_dtype d) {
+  return d == HB_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : d == HB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+}
+
+// 2-D row-major [rows, cols] tensor of a 16-bit type, box [box_rows, 64 cols], 128-byte swizzle.
 // heads > 0: that many such tensors `step` elements apart, rows of ld elements.
-static int encode_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int box_rows, int heads = 0, int64_t ld = 0,
-                      int64_t step = 0) {
+static int encode_map(CUtensorMap* tm, const void* ptr, hb_dtype dtype, int64_t rows, int64_t cols, int box_rows, int heads = 0,
+                      int64_t ld = 0, int64_t step = 0) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return fail(HB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)heads};
   cuuint64_t strides[2] = {(cuuint64_t)(heads ? ld : cols) * 2, (cuuint64_t)step * 2};
   cuuint32_t box[3] = {(cuuint32_t)kTileK, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, heads ? 3 : 2, const_cast<void*>(ptr), dims, strides,
+  CUresult r = enc(tm, tm_type(dtype), heads ? 3 : 2, const_cast<void*>(ptr), dims, strides,
                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(HB_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
   return HB_OK;
 }
 
-// Output map: [rows, cols] elements of elt bytes, row stride ld elements, box
+// Output map: [rows, cols] elements, row stride ld elements, box
 // [box_rows, 128 cols], no swizzle (the kernel stages rows of 128 features densely).
 // heads > 0: that many such tensors `step` elements apart.
-static int encode_out_map(CUtensorMap* tm, void* ptr, int64_t rows, int64_t cols, int64_t ld, bool f32,
+static int encode_out_map(CUtensorMap* tm, void* ptr, hb_dtype dtype, int64_t rows, int64_t cols, int64_t ld,
                           int box_rows, int heads = 0, int64_t step = 0) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return fail(HB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  const cuuint64_t elt = f32 ? 4 : 2;
+  const cuuint64_t elt = dtype_size(dtype);
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)heads};
   cuuint64_t strides[2] = {(cuuint64_t)ld * elt, (cuuint64_t)step * elt};
   cuuint32_t box[3] = {(cuuint32_t)kTileN, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, heads ? 3 : 2, ptr, dims,
-                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+  CUresult r = enc(tm, tm_type(dtype), heads ? 3 : 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(HB_ERR_CUDA, "cuTensorMapEncodeTiled (output) failed with code %d", (int)r);
   return HB_OK;
@@ -950,7 +954,7 @@ static int encode_out_map(CUtensorMap* tm, void* ptr, int64_t rows, int64_t cols
 bool gemm_tc_supported(int64_t M, int64_t N, int64_t K, hb_dtype dtype) {
   // K need not fill its last 64-wide chunk: the tensor maps deliver zeros past the end of a row
   // (rows must be 16-byte multiples)
-  return dtype == HB_BF16 && M >= 1 && N >= 1 && K >= 8 && K % 8 == 0 &&
+  return (dtype == HB_BF16 || dtype == HB_F16) && M >= 1 && N >= 1 && K >= 8 && K % 8 == 0 &&
          N < (1ll << 30) && M < (1ll << 30);
 }
 
@@ -983,8 +987,9 @@ static int pick_cluster_splits(int units, int k_chunks, int sm_count) {
 }
 
 int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int64_t N, int64_t K,
-                 int epilogue, bool out_f32, int device, int force_splits, const TcGroups* groups, const TcHeads* heads) {
-  if (!gemm_tc_supported(M, N, K, HB_BF16))
+                 int epilogue, bool out_f32, int device, int force_splits, const TcGroups* groups, const TcHeads* heads,
+                 hb_dtype dtype) {
+  if (!gemm_tc_supported(M, N, K, dtype) || (dtype == HB_F16 && (groups || heads || epilogue == kEpiAct || epilogue == kEpiPush || epilogue == kEpiResidual)))
     return fail(HB_ERR_INVALID_ARG, "gemm_tc: unsupported shape M=%lld N=%lld K=%lld", (long long)M,
                 (long long)N, (long long)K);
   if ((reinterpret_cast<uintptr_t>(X) & 15) || (reinterpret_cast<uintptr_t>(W) & 15))
@@ -997,6 +1002,7 @@ int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int6
                 device, di.cc_major, di.cc_minor);
   TcGemmPlan& pl = *plan;
   pl.M = M; pl.K = K;
+  pl.dtype = dtype;
   pl.epilogue = epilogue;
   pl.out_f32 = out_f32;
   pl.groups = groups ? groups->groups : 0;
@@ -1178,16 +1184,16 @@ int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int6
     if (cur >= 0 && cur < 64 && !dev_done[cur]) {
       // 227 KiB per CTA minus the kernel's static shared memory (barriers, flags, row scales)
       for (auto* k : {gemm_tc_kernel<false, false, false>, gemm_tc_kernel<false, true, false>, gemm_tc_kernel<true, true, false>,
-                      gemm_tc_kernel<false, false, true>})
+                      gemm_tc_kernel<false, false, true>, gemm_tc_kernel<false, false, false, __half>})
         HB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
       dev_done[cur] = true;
     }
   }
-  rc = encode_map(&pl.tm_w, W, groups ? N * groups->groups : heads ? N * heads->heads : N, K, kTileN);
+  rc = encode_map(&pl.tm_w, W, dtype, groups ? N * groups->groups : heads ? N * heads->heads : N, K, kTileN);
   if (rc) return rc;
-  if (heads) return encode_map(&pl.tm_x, X, M, K, pl.m_pad, heads->heads, heads->ldx, heads->x_step);
-  rc = encode_map(&pl.tm_x, X, M, groups ? pl.ldx : K, pl.m_pad);
-  if (!rc && pl.N2) rc = encode_map(&pl.tm_w2, groups->shared_w, groups->shared_n, pl.K2, kTileN);
+  if (heads) return encode_map(&pl.tm_x, X, dtype, M, K, pl.m_pad, heads->heads, heads->ldx, heads->x_step);
+  rc = encode_map(&pl.tm_x, X, dtype, M, groups ? pl.ldx : K, pl.m_pad);
+  if (!rc && pl.N2) rc = encode_map(&pl.tm_w2, groups->shared_w, dtype, groups->shared_n, pl.K2, kTileN);
   return rc;
 }
 
@@ -1268,8 +1274,8 @@ int gemm_tc_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, voi
     const int box_rows = pl.cluster ? pl.m_pad / pl.splits : 16;
     // groups of different widths share the rows: columns between one's width and the next
     // multiple of 128 may be written, and every reader of them multiplies them by zero
-    int rc = encode_out_map(&tm_y, Y, pl.M, pl.groups ? std::min(ldy, std::max(pl.N, pl.N2)) : pl.N, ldy, pl.out_f32, box_rows,
-                            pl.heads.heads, pl.heads.y_step);
+    int rc = encode_out_map(&tm_y, Y, pl.out_f32 ? HB_F32 : pl.dtype, pl.M,
+                            pl.groups ? std::min(ldy, std::max(pl.N, pl.N2)) : pl.N, ldy, box_rows, pl.heads.heads, pl.heads.y_step);
     if (rc) return rc;
   }
   CUtensorMap tm_h;
@@ -1283,9 +1289,9 @@ int gemm_tc_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, voi
       return fail(HB_ERR_INVALID_ARG, "gemm_tc: the residual epilogue needs a cluster plan, bf16 output and a norm link");
     if ((reinterpret_cast<uintptr_t>(link->resid) & 15) || link->rowsq_stride < pl.n_tiles)
       return fail(HB_ERR_INVALID_ARG, "gemm_tc: bad residual buffer or row-sum stride");
-    int rc = encode_out_map(&tm_h, link->resid, pl.M, pl.N, ldy, false, pl.m_pad / pl.splits);
+    int rc = encode_out_map(&tm_h, link->resid, pl.dtype, pl.M, pl.N, ldy, pl.m_pad / pl.splits);
     if (rc) return rc;
-    p.norm_w = (const __nv_bfloat16*)link->norm_w;
+    p.norm_w = link->norm_w;
     p.rowsq_out = link->rowsq_out;
     p.rowsq_stride = link->rowsq_stride;
   }
@@ -1302,8 +1308,8 @@ int gemm_tc_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, voi
       return fail(HB_ERR_INVALID_ARG, "gemm_tc: the RoPE epilogue needs a cluster plan over [q|k|v] heads of 128");
     p.rope_cs = link->rope_cs;
     p.kv_slots = link->kv_slots;
-    p.k_cache = (__nv_bfloat16*)link->k_cache;
-    p.v_cache = (__nv_bfloat16*)link->v_cache;
+    p.k_cache = link->k_cache;
+    p.v_cache = link->v_cache;
     p.rope_nq = link->n_q_heads;
     p.rope_nkv = link->n_kv_heads;
     p.kv_num_blocks = link->num_blocks;
@@ -1350,7 +1356,9 @@ int gemm_tc_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, voi
   cfg.attrs = attr;
   cfg.numAttrs = na;
   const bool general = !pl.act.silu() || pl.gate_bias || pl.up_bias || pl.epilogue == kEpiAct;
-  auto* kernel = pl.groups ? gemm_tc_kernel<true, true, false>
+  if (pl.dtype == HB_F16 && general) return fail(HB_ERR_INVALID_ARG, "gemm_tc: f16 has plain outputs and SwiGLU only");
+  auto* kernel = pl.dtype == HB_F16 ? gemm_tc_kernel<false, false, false, __half>
+                 : pl.groups ? gemm_tc_kernel<true, true, false>
                  : pl.heads.heads ? gemm_tc_kernel<false, false, true>
                  : general ? gemm_tc_kernel<false, true, false> : gemm_tc_kernel<false, false, false>;
   HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, pl.tm_w, pl.tm_x, tm_y, tm_h, p));

@@ -182,7 +182,7 @@ int hb_gemm_heads(void* stream, void* Y, const void* X, const void* W, int64_t M
   h.heads = heads; h.ldx = ldx; h.x_step = x_step; h.ldy = ldy; h.y_step = y_step;
   auto st = (cudaStream_t)stream;
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  if (M && hb::gemm_tc_supported(M, N, K, dtype) && hb::gemm_tc_heads_supported(N, K, false, h) && al(X) && al(W) && al(Y)) {
+  if (M && dtype == HB_BF16 && hb::gemm_tc_supported(M, N, K, dtype) && hb::gemm_tc_heads_supported(N, K, false, h) && al(X) && al(W) && al(Y)) {
     int dev = 0;
     HB_CUDA_CHECK(cudaGetDevice(&dev));
     hb::TcGemmPlan plan;
@@ -275,7 +275,7 @@ int hb_gemm_grouped(void* stream, void* Y, const void* X, const void* W, const h
   const hb::TcGroups g = groups_of(p);
   const int64_t M = (int64_t)p->max_tiles * p->m_pad;
   auto st = (cudaStream_t)stream;
-  if (hb::gemm_tc_supported(M, p->N, p->K, dtype) && p->m_pad % 16 == 0) {
+  if (dtype == HB_BF16 && hb::gemm_tc_supported(M, p->N, p->K, dtype) && p->m_pad % 16 == 0) {
     int dev = 0;
     HB_CUDA_CHECK(cudaGetDevice(&dev));
     hb::TcGemmPlan plan;

@@ -4,6 +4,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.h"
 
 namespace hb {
@@ -148,9 +150,11 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   d |= (uint64_t)2 << 61;                        // layout type: 128-byte swizzle
   return d;
 }
-// Instruction descriptor: bf16 x bf16 -> f32, A and B K-major, M = 128, N = n.
+// Instruction descriptor: T x T -> f32 (bf16 or f16), A and B K-major, M = 128, N = n.
+template <typename T = __nv_bfloat16>
 __device__ __forceinline__ uint32_t make_idesc(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+  constexpr uint32_t fmt = std::is_same<T, __half>::value ? 0u : 1u;
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(kTileN >> 4) << 24);
 }
 
