@@ -35,6 +35,7 @@
 #include "comm.h"
 #include "common.h"
 #include "gemm.h"
+#include "gemm_act.cuh"
 #include "peer_sync.cuh"
 #include "tc_core.cuh"
 
@@ -160,53 +161,6 @@ __device__ __forceinline__ void push_tile(const TcParams& p, const uint8_t* stag
     peer_st_release(&reinterpret_cast<CommFlags*>(p.push_peer[q])->tflag[(row_block * R + me) * T + ti], seq + 1);
 }
 
-// Standard normal distribution function by formula 7.1.26 of Abramowitz and Stegun, Handbook of
-// Mathematical Functions, for erfc (within 1.5e-7 of the exact value), without branches.
-__device__ __forceinline__ float normal_cdf(float g) {
-  const float a = fabsf(g) * 0.70710678f;
-  const float t = __fdividef(1.f, fmaf(0.3275911f, a, 1.f));
-  float p = fmaf(1.061405429f, t, -1.453152027f);
-  p = fmaf(p, t, 1.421413741f);
-  p = fmaf(p, t, -0.284496736f);
-  p = fmaf(p, t, 0.254829592f);
-  const float half_erfc = 0.5f * p * t * __expf(-a * a);
-  return g < 0.f ? half_erfc : 1.f - half_erfc;
-}
-
-// An activation without a gate, on 16 outputs: the form is looked up once.
-__device__ __forceinline__ void single_16(float (&v)[16], const GatedAct& act) {
-  if (act.form == GatedAct::kErf) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float g = fminf(v[j], act.limit);
-      v[j] = g * normal_cdf(g);
-    }
-  } else if (act.form == GatedAct::kTanh) {
-    const float k = __fdividef(2.f, act.limit);
-#pragma unroll
-    for (int j = 0; j < 16; ++j)  // tanh(y) = 1 - 2 / (1 + e^2y)
-      v[j] = act.limit - __fdividef(2.f * act.limit, 1.f + __expf(fminf(v[j] * k, 80.f)));
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float g = fminf(v[j], act.limit), z = act.slope * fmaf(act.cubic * g * g, g, g);
-      v[j] = z < -80.f ? 0.f : __fdividef(g, 1.f + __expf(-z));
-    }
-  }
-}
-
-// Gated activation of one output element (fast divide and exponential, as silu_f).
-template <bool GENERAL>
-__device__ __forceinline__ float gated_f(float g, float u, const GatedAct& act) {
-  if (!GENERAL) return silu_f(g) * u;
-  g = fminf(g, act.limit);
-  u = fminf(fmaxf(u, -act.limit), act.limit);
-  if (act.form == GatedAct::kErf) return g * normal_cdf(g) * (u + act.shift);
-  const float z = act.slope * fmaf(act.cubic * g * g, g, g);
-  // far below zero the gate is zero (the fast divide wants a denominator below 2^126)
-  return z < -80.f ? 0.f : __fdividef(g, 1.f + __expf(-z)) * (u + act.shift);
-}
-
 // ----------------------------------------------------------------------- kernel
 // GROUPS: rows sorted by group (TcGroups).  GENERAL: any GatedAct and biases of the pair, else SiLU.
 // HEADS: blockIdx.z counts independent products (TcHeads).  The instance without any of them is the
@@ -315,7 +269,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   TC_TRACE(tid == 0, 1);
   // (The next kernel is released once this CTA's accumulator is complete, below, not here: its
   // CTAs hold their pipeline's shared memory from the moment they are resident.)
-  if (!(warp == 0 && lane == 0)) pdl_wait();  // the producer waits after its weight prefetch
+  if (warp != 0) pdl_wait();  // the producer waits after its weight prefetch
 
   if (warp >= 2 && p.rowsq_in) {
     // deferred norm: scale of every batch row of this tile column, from the row sums the
@@ -360,111 +314,113 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       s_pscale[i] = m < p.M ? __ldcg(p.post_scale + (int64_t)m * p.post_groups + grp) : 0.f;
     }
   }
+  // Producer and issuer run in their whole warp (see elect_one); the stage and its parity are counted, not divided.
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------------------------------------------------- TMA producer
-      int armed = 0;  // k-chunks whose copies were issued
-      const uint64_t w_policy = l2_policy_evict_first();
-      // every weight byte is read once per launch: it may leave L2 first (measured +1 % on the
-      // 8B decode step against the default policy)
-      auto load_w = [&](uint32_t dst, int kx, int row, uint32_t bar) {
-        tma_load_2d_hint(dst, w_map, kx, row, bar, w_policy);
-      };
-      auto load_x = [&](uint32_t dst, int kx, uint32_t bar) {
-        if (HEADS) tma_load_3d(dst, &tm_x, kx, m_tile * p.m_pad, head, bar);
-        else tma_load_2d(dst, &tm_x, kx, m_tile * p.m_pad, bar);
-      };
-      // Weights never depend on the previous kernel: the first stages' weight slabs are
-      // requested before waiting for it; activations only afterwards.
-      const int pre = min(p.stages, n_kc);
-      for (int i = 0; i < pre; ++i) {
-        const uint32_t full = smem_u32(&s_full[i]);
-        const uint32_t sa = smem_base + i * stage_bytes;
-        mbar_expect_tx(full, stage_bytes);
-        const int kx = (kc0 + i) * kTileK;
-        load_w(sa, kx, w_row, full);
-        if (swiglu) load_w(sa + a_bytes, kx, up_row_offset + w_row, full);
-      }
-      // (Requesting further chunks into L2 at this point was measured harmful: -2 % to -7 % per
-      // decode step after HBM-bound kernels, no gain after an NVLink exchange.  Requesting the
-      // NEXT kernel's weights into L2 once this CTA has issued its last load, so that HBM works
-      // through the tail (a linear prefix of 8-32 MB, or per CTA of the next kernel the 1-4
-      // chunks after the stages it fetches by itself): within +-0.4 % per step, -1.5 % and worse
-      // from 8 chunks or 64 MB: neither the tail nor the restart of the stream waits for HBM.  With the weights already resident in L2 the 8B q|k|v projection takes
-      // 15.7 us instead of 17.6: the time is L2-to-SM transport and the serial chain of the tail.)
-      pdl_wait();
-      TC_LAUNCH_TRACE(3);
-      for (int i = 0; i < pre; ++i) {
-        load_x(smem_base + i * stage_bytes + a_bytes * n_acc, (kc0 + i) * kTileK, smem_u32(&s_full[i]));
-      }
-      armed = pre;
-      for (int i = pre; i < n_kc; ++i) {
-        const int s = i % p.stages;
-        const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
-        if (!mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, &s_abort)) break;
-        const uint32_t full = smem_u32(&s_full[s]);
-        const uint32_t sa = smem_base + s * stage_bytes;
-        mbar_expect_tx(full, stage_bytes);
-        const int kx = (kc0 + i) * kTileK;
-        load_w(sa, kx, w_row, full);
-        if (swiglu) load_w(sa + a_bytes, kx, up_row_offset + w_row, full);
-        load_x(sa + a_bytes * n_acc, kx, full);
-        armed = i + 1;
-      }
-      if (s_abort) {
-        // let every issued copy land before this CTA's shared memory can be reused
-        for (int i = max(0, armed - p.stages); i < armed; ++i) {
-          const int s = i % p.stages;
-          const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
-          for (uint32_t it = 0; it < kSpinLimit && !mbar_try(smem_u32(&s_full[s]), ph); ++it) {
-          }
+    // ------------------------------------------------------------ TMA producer
+    const uint32_t e = elect_one();
+    const uint64_t w_policy = l2_policy_evict_first();
+    // every weight byte is read once per launch: it may leave L2 first (measured +1 % on the
+    // 8B decode step against the default policy)
+    auto load_w = [&](uint32_t dst, int kx, int row, uint32_t bar) {
+      tma_load_2d_hint_if(e, dst, w_map, kx, row, bar, w_policy);
+    };
+    auto load_x = [&](uint32_t dst, int kx, uint32_t bar) {
+      if (HEADS) tma_load_3d_if(e, dst, &tm_x, kx, m_tile * p.m_pad, head, bar);
+      else tma_load_2d_if(e, dst, &tm_x, kx, m_tile * p.m_pad, bar);
+    };
+    // Weights never depend on the previous kernel: the first stages' weight slabs are
+    // requested before waiting for it; activations only afterwards.
+    const int pre = min(p.stages, n_kc);
+    for (int i = 0; i < pre; ++i) {
+      const uint32_t full = smem_u32(&s_full[i]);
+      const uint32_t sa = smem_base + i * stage_bytes;
+      mbar_expect_tx_if(e, full, stage_bytes);
+      const int kx = (kc0 + i) * kTileK;
+      load_w(sa, kx, w_row, full);
+      if (swiglu) load_w(sa + a_bytes, kx, up_row_offset + w_row, full);
+    }
+    // (Requesting further chunks into L2 at this point was measured harmful: -2 % to -7 % per
+    // decode step after HBM-bound kernels, no gain after an NVLink exchange.  Requesting the
+    // NEXT kernel's weights into L2 once this CTA has issued its last load, so that HBM works
+    // through the tail (a linear prefix of 8-32 MB, or per CTA of the next kernel the 1-4
+    // chunks after the stages it fetches by itself): within +-0.4 % per step, -1.5 % and worse
+    // from 8 chunks or 64 MB: neither the tail nor the restart of the stream waits for HBM.  With the weights already resident in L2 the 8B q|k|v projection takes
+    // 15.7 us instead of 17.6: the time is L2-to-SM transport and the serial chain of the tail.)
+    pdl_wait();
+#ifdef HB_TC_TRACE
+    if (e) tc_launch_trace(p.trace_id, 3, p.N, p.k_chunks * kTileK);
+#endif
+    for (int i = 0; i < pre; ++i) {
+      load_x(smem_base + i * stage_bytes + a_bytes * n_acc, (kc0 + i) * kTileK, smem_u32(&s_full[i]));
+    }
+    int armed = pre;  // k-chunks whose copies were issued
+    int s = pre == p.stages ? 0 : pre;
+    uint32_t ph = 0;
+    for (int i = pre; i < n_kc; ++i) {
+      if (!mbar_wait(smem_u32(&s_empty[s]), ph, &s_abort)) break;
+      const uint32_t full = smem_u32(&s_full[s]);
+      const uint32_t sa = smem_base + s * stage_bytes;
+      mbar_expect_tx_if(e, full, stage_bytes);
+      const int kx = (kc0 + i) * kTileK;
+      load_w(sa, kx, w_row, full);
+      if (swiglu) load_w(sa + a_bytes, kx, up_row_offset + w_row, full);
+      load_x(sa + a_bytes * n_acc, kx, full);
+      armed = i + 1;
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
+    }
+    if (s_abort) {
+      // let every issued copy land before this CTA's shared memory can be reused
+      for (int i = max(0, armed - p.stages); i < armed; ++i) {
+        const uint32_t full = smem_u32(&s_full[i % p.stages]), par = (uint32_t)(i / p.stages) & 1u;
+        for (uint32_t it = 0; it < kSpinLimit && !mbar_try(full, par); ++it) {
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------ MMA issuer
-      const uint32_t idesc = make_idesc<T>(p.m_pad);
-      bool ok = true;
-      for (int i = 0; i < n_kc && ok; ++i) {
-        const int s = i % p.stages;
-        const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
-        ok = mbar_wait(smem_u32(&s_full[s]), ph, &s_abort);
-        if (!ok) break;
-        TC_TRACE(i == 0, 2);
-        tc_fence_after();
-        const uint32_t sa = smem_base + s * stage_bytes;
-        const uint64_t b_desc = make_smem_desc(sa + a_bytes * n_acc);
+    // -------------------------------------------------------------- MMA issuer
+    const uint32_t e = elect_one();
+    const uint32_t idesc = make_idesc<T>(p.m_pad);
+    const uint64_t a0 = make_smem_desc(smem_base), b0 = make_smem_desc(smem_base + a_bytes * n_acc);
+    const uint32_t step = stage_bytes >> 4;  // of a descriptor, from stage to stage
+    const uint32_t acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+    bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
+    for (int i = 0; i < n_kc; ++i) {
+      ok = mbar_wait(smem_u32(&s_full[s]), ph, &s_abort);
+      if (!ok) break;
+      TC_TRACE(lane == 0 && i == 0, 2);
+      tc_fence_after();
+      const uint64_t b_desc = b0 + (uint64_t)(s * step);
 #pragma unroll
-        for (int acc = 0; acc < 2; ++acc) {
-          if (acc < n_acc) {
-            const uint64_t a_desc = make_smem_desc(sa + acc * a_bytes);
+      for (int acc = 0; acc < 2; ++acc) {
+        if (acc < n_acc) {
+          const uint64_t a_desc = a0 + (uint64_t)(s * step + acc * (a_bytes >> 4));
 #pragma unroll
-            for (int k = 0; k < kTileK / kUmmaK; ++k) {
-              // advancing K by 16 elements = 32 bytes inside the swizzled row
-              umma_bf16(tmem_base + acc * p.m_pad, a_desc + (uint64_t)(k * 2),
-                        b_desc + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-            }
+          for (int k = 0; k < kTileK / kUmmaK; ++k) {
+            // advancing K by 16 elements = 32 bytes inside the swizzled row
+            umma_if(e, acc0 + acc * p.m_pad, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc,
+                    (i > 0 || k > 0) ? 1u : 0u);
           }
         }
-        tc_commit(smem_u32(&s_empty[s]));  // frees the stage once these MMAs have read it
       }
-      // only this thread polls for the accumulator; the other 127 sleep at the CTA
-      // barrier below
-      if (ok) {
-        tc_commit(smem_u32(&s_done));
-        ok = mbar_wait(smem_u32(&s_done), 0, &s_abort);
-      }
-      if (!ok) s_abort = 1;
-      // The next kernel may become resident now: it requests its first weight stages while this
-      // kernel exchanges, sums and stores, i.e. while HBM would otherwise idle.  Releasing it at
-      // the start of this kernel instead (resident and holding shared memory for the whole
-      // stream) measured 4.36 against 4.32 ms per 8B decode step; after the last load was
-      // issued, or half-way through the stream, in between.
-      pdl_launch_dependents();
-      TC_TRACE(true, 3);
+      tc_commit_if(e, smem_u32(&s_empty[s]));  // frees the stage once these MMAs have read it
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
+    // only this warp polls for the accumulator; the others sleep at the CTA barrier below
+    if (ok) {
+      tc_commit_if(e, smem_u32(&s_done));
+      ok = mbar_wait(smem_u32(&s_done), 0, &s_abort);
+    }
+    if (!ok) s_abort = 1;
+    // The next kernel may become resident now: it requests its first weight stages while this
+    // kernel exchanges, sums and stores, i.e. while HBM would otherwise idle.  Releasing it at
+    // the start of this kernel instead (resident and holding shared memory for the whole
+    // stream) measured 4.36 against 4.32 ms per 8B decode step; after the last load was
+    // issued, or half-way through the stream, in between.
+    pdl_launch_dependents();
+    TC_TRACE(lane == 0, 3);
     __syncwarp();
   }
 

@@ -110,18 +110,61 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+// One lane of a converged warp, the same one every time.
+//
+// The loops that feed the tensor cores run in the whole warp, and only the instructions that must be
+// issued once are predicated on this: what they take (descriptors, coordinates, barriers) then stays in
+// uniform registers.  Inside `if (lane == 0)` every one of them moves its operands over first; an MMA
+// took 62 cycles to issue and a chunk of 64 channels 585, whatever the tile's width.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e;
+}
+// Predicated on `e`: arrive and expect bytes; loads; MMA; commit.
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t e, uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
+               ::"r"(bar), "r"(bytes), "r"(e)
                : "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc], bf16 inputs, fp32 accumulate.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tma_load_2d_if(uint32_t e, uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t bar) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
+      ::"r"(dst), "l"(tm), "r"(x), "r"(y), "r"(bar), "r"(e)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_hint_if(uint32_t e, uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t bar,
+                                                    uint64_t policy) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%2, %3}], [%4], %5;\n\t}"
+      ::"r"(dst), "l"(tm), "r"(x), "r"(y), "r"(bar), "l"(policy), "r"(e)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_if(uint32_t e, uint32_t dst, const CUtensorMap* tm, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}"
+      ::"r"(dst), "l"(tm), "r"(x), "r"(y), "r"(z), "r"(bar), "r"(e)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t e, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(e)
+      : "memory");
+}
+// D[tmem] (+)= A[smem desc] * B[smem desc], 16-bit inputs, fp32 accumulate.
+__device__ __forceinline__ void umma_if(uint32_t e, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(e)
       : "memory");
 }
 // 32 lanes x 16 consecutive fp32 columns: thread i gets lane (base_lane + i).
