@@ -35,6 +35,78 @@ def test_probabilities_match_the_oracle(hb, cuda, vocab, temperature, top_p):
             assert np.max(np.abs(got[i][same] - want[same])) <= 1e-3 * float(want.max()) + (0.0 if len(diff) == 0 else 1e-2)
 
 
+def nucleus_in_64_bits(z, top_p):
+    """Softmax, and the sum of it down to the last token of the nucleus, in fp64."""
+    e = np.exp(z.astype(np.float64) - z.max())
+    p = e / e.sum()
+    order = np.argsort(-p, kind="stable")
+    last = min(int(np.searchsorted(np.cumsum(p[order]), top_p)), len(p) - 1)
+    kept = p >= p[order[last]]
+    return p, kept, order, last
+
+
+# one CTA per 4096 tokens up to eight, slices of whole vectors or not, and above 409600 one CTA per row
+@pytest.mark.parametrize("vocab", [1, 3, 4095, 4096, 4097, 8193, 16388, 32001, 409600, 409603])
+@pytest.mark.parametrize("top_p", [1.0, 0.97, 1e-6])
+@pytest.mark.parametrize("shape", ["steep", "flat", "ties", "masked"])
+def test_rows_of_every_size(hb, cuda, vocab, top_p, shape):
+    """Error of a probability of logit z below the row's maximum: the fast exponential is within 2 + 1.173 |z| ulp (its stated
+    bound), its argument and the penalties are rounded (1 ulp of |z| < 64 each: |z| and 2 ulp of the result), and the factors
+    that follow: 2^-23 (8 + 3.2 |z|); the one-CTA form adds two fp32 sums of vocab / 1024 numbers per thread.  Tokens whose cumulative mass lies within the rounding of the sum may be in or out."""
+    rng = np.random.default_rng(vocab)
+    sums = vocab / 1024 + 10 if vocab > 409600 else 0
+    n = 2
+    z = rng.standard_normal((n, vocab)).astype(np.float32) * {"steep": 4.0, "flat": 0.0, "ties": 2.0, "masked": 1.0}[shape]
+    if shape == "ties":
+        z = np.round(z)
+    if shape == "masked":
+        z[:, rng.random(vocab) < 0.9] = -np.inf
+        z[:, vocab // 2] = 0.0
+    counts = np.zeros((n, vocab), dtype=np.int32)
+    counts[:, :: 7] = 2
+    seeds = np.arange(1, n + 1, dtype=np.int64)
+    for c in (None, torch.from_numpy(counts).to(cuda)):
+        tokens, probs = hb.sample(torch.from_numpy(z).to(cuda), torch.from_numpy(seeds).to(cuda), 1.0, top_p, c, 0.5, 0.25)
+        tokens, probs = tokens.cpu().numpy(), probs.cpu().numpy().astype(np.float64)
+        for i in range(n):
+            zi = z[i]
+            if c is not None:
+                f = counts[i].astype(np.float32)
+                zi = np.where(f > 0, zi - np.float32(0.5) - np.float32(0.25) * (f / np.float32(max(f.sum(), 1))), zi).astype(np.float32)
+            p, kept, order, last = nucleus_in_64_bits(zi, top_p)
+            got = probs[i] > 0
+            if top_p < 1:
+                differ = got != (kept & (p > 1e-37))
+                cum = np.cumsum(p[order])
+                edge = np.abs(cum - top_p) < 2.0 ** -20
+                assert not differ.any() or edge[max(0, last - 1):last + 2].any(), np.nonzero(differ)[0][:5]
+                p = np.where(got, p, 0.0)
+                p /= p.sum()
+            far = np.where(np.isfinite(zi), zi.max() - zi.astype(np.float64), 0.0)
+            assert np.all(np.abs(probs[i] - p) <= 2.0 ** -23 * (8 + 3.2 * far + sums) * p + 1e-37)
+            assert probs[i][tokens[i]] > 0
+            c64, u = np.cumsum(probs[i]), S.uniform_from_seed(int(seeds[i]))
+            t = int(tokens[i])
+            assert c64[t] >= u * c64[-1] - 1e-5 and (t == 0 or c64[t - 1] <= u * c64[-1] + 1e-5)
+
+
+@pytest.mark.parametrize("vocab", [40, 50000])
+def test_rows_without_a_maximum(hb, cuda, vocab):
+    """Nothing but masked tokens, or a NaN, or +inf: no numbers without a nucleus, zeros with one, token 0."""
+    z = torch.zeros(3, vocab, device=cuda)
+    z[0] = -float("inf")
+    z[1, vocab // 2] = float("nan")
+    z[2, vocab // 3] = float("inf")
+    seeds = torch.arange(3, device=cuda)
+    for top_p in (1.0, 0.9):
+        tokens, probs = hb.sample(z, seeds, 1.0, top_p)
+        assert tokens.tolist() == [0, 0, 0]
+        if top_p < 1:
+            assert not probs.any()
+        else:
+            assert bool(probs.isnan().all(dim=1)[:2].all()) and bool(probs[2, vocab // 3].isnan())
+
+
 def test_known_answers_on_the_device(hb, cuda, kats):
     case = kats["sampling"]["nucleus_filter_keeps_top_mass"]
     logits = np.log(np.array([case["probs"]], dtype=np.float32))

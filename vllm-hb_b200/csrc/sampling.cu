@@ -3,15 +3,22 @@
 // src/sampling/penalty.rs:28-52; apply_temperature / softmax_inplace / nucleus_filter /
 // renormalize, src/sampling/nucleus.rs:7-62), for a whole batch of logit rows at once.
 // The reference copies every [vocab] logit row to the host and sorts it there; here the
-// probabilities never leave the device: one CTA per row, the row streamed from L2, and
-// the nucleus found as a probability threshold by bisection instead of a sort.
+// probabilities never leave the device, and the nucleus is found as a probability threshold
+// instead of by a sort.  All arithmetic is fp32 as in the reference.
 //
-// A row is read a few dozen times (513 KB at the Llama-3 vocabulary: L2-resident), so the
-// kernels are latency-, not HBM-bound; all arithmetic is fp32 as in the reference.
+// A cluster of up to eight CTAs takes a row: every CTA keeps its slice of the probabilities in shared
+// memory, so that logits are read and results written once, and what the row has in common (maximum,
+// sum, masses above a threshold) goes through the partners' shared memory.  The number of CTAs
+// follows from the vocabulary alone, so that a row's result does not depend on its batch.  64 rows of
+// 128256 with a nucleus: 81 us; with one CTA per row and a bisection of forty passes over
+// the row in L2: 518 us.  Bound: the barriers of the cluster, about ten of them one after another.
+// Vocabularies whose slices leave shared memory (above 409600) take the one-CTA form.
 #include <cfloat>
 #include <climits>
+#include <mutex>
 
 #include "common.h"
+#include "tc_core.cuh"
 
 namespace hb {
 
@@ -46,6 +53,7 @@ __device__ __forceinline__ float uniform_from_seed(uint64_t seed) {
   return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
+// One CTA per row, any vocabulary.
 __global__ void __launch_bounds__(kSampleThreads)
 sample_kernel(const SampleParams p) {
   __shared__ float s_red[33];
@@ -181,6 +189,361 @@ sample_kernel(const SampleParams p) {
   }
 }
 
+// ------------------------------------------------------------------ a cluster per row
+constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32;
+constexpr int kRowCtas = 8;      // of a cluster, at most
+constexpr int kCuts = 7;         // thresholds tried per pass over the slice
+constexpr int kBandCap = 256;    // probabilities that one CTA ranks by itself
+constexpr int kSliceCap = 51200; // of a slice, in shared memory
+
+struct RowShared {
+  float v[2][kRowCtas][2 * kCuts];        // what the partners bring to an exchange; two, used in turn
+  double total[2][kRowCtas];              // sums of the partners: of all, of the kept tokens
+  unsigned long long n[kRowCtas];
+  float warp_part[kRowWarps][2 * kCuts];
+  float band[kBandCap];
+  float thr;
+  int n_band;
+  int warp_arg[kRowWarps];
+  int arg[kRowCtas];
+  double mass[kRowWarps];                 // of every warp's part of the slice
+};
+
+__device__ __forceinline__ void st_cluster_u64(uint32_t caddr, unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(caddr), "l"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster_f64(uint32_t caddr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(caddr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t caddr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(caddr), "r"(v) : "memory");
+}
+
+// Exchanges N numbers per CTA: afterwards every CTA holds all of them in s.v[turn].  `mine` (of every
+// thread) are the CTA's own.  The buffers are used in turn: whoever writes one again has passed the
+// barrier that its readers reach after reading it.
+template <int N>
+__device__ __forceinline__ const float (*exchange(RowShared& s, int& turn, const float (&mine)[N], int rank, int ctas))[2 * kCuts] {
+  turn ^= 1;
+  const int tid = threadIdx.x;
+  if (tid < ctas) {
+    const uint32_t dst = cluster_map(smem_u32(&s.v[turn][rank][0]), tid);
+#pragma unroll
+    for (int i = 0; i < N; ++i) st_cluster_f32(dst + 4 * i, mine[i]);
+  }
+  cluster_sync_all();
+  return s.v[turn];
+}
+
+// Sums over the CTA of N numbers per thread, in a fixed order; every thread gets them.
+template <int N>
+__device__ __forceinline__ void cta_sums(RowShared& s, float (&v)[N]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = warp_sum(v[i]);
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) s.warp_part[warp][i] = v[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float t = lane < kRowWarps ? s.warp_part[lane][i] : 0.f;
+    v[i] = warp_sum(t);
+  }
+  __syncthreads();
+}
+// Sum over the row of one number per lane, in a fixed order; s.mass keeps the warps', s.total[which] the CTAs'.
+__device__ __forceinline__ double row_sum(RowShared& s, int which, double v, int rank, int ctas) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) s.mass[warp] = v;
+  __syncthreads();
+  if (tid < ctas) {
+    v = 0.0;
+    for (int w = 0; w < kRowWarps; ++w) v += s.mass[w];
+    st_cluster_f64(cluster_map(smem_u32(&s.total[which][rank]), tid), v);
+  }
+  cluster_sync_all();
+  v = 0.0;
+  for (int r = 0; r < ctas; ++r) v += s.total[which][r];
+  return v;
+}
+
+__global__ void __launch_bounds__(kRowThreads)
+sample_row_kernel(const SampleParams p, int slice, int wide) {
+  extern __shared__ __align__(16) float s_q[];  // this CTA's part of the row
+  __shared__ RowShared s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ctas = (int)gridDim.x, rank = (int)blockIdx.x;  // grid.x = the cluster
+  const int64_t row = blockIdx.y, V = p.vocab;
+  const int64_t first = min(V, (int64_t)rank * slice);
+  const int n = (int)(min(V, first + slice) - first);
+  const float* x = p.logits + row * V + first;
+  const uint32_t* cnt = p.counts ? p.counts + row * V + first : nullptr;
+  float* pr = p.probs + row * V + first;
+  const bool penal = cnt && (fabsf(p.presence) >= 1e-6f || fabsf(p.frequency) >= 1e-6f);
+  if (tid == 0) s.n_band = 0;
+  int turn = 0;
+  cluster_sync_all();  // the partners have started: their shared memory may be written
+  float total_f = 1.f;
+  if (penal) {
+    // tokens seen so far, a whole number
+    __shared__ unsigned long long s_sum[kRowWarps];
+    unsigned long long t = 0;
+    for (int i = tid; i < n; i += kRowThreads) t += cnt[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) s_sum[warp] = t;
+    __syncthreads();
+    if (tid < ctas) {
+      t = 0;
+      for (int w = 0; w < kRowWarps; ++w) t += s_sum[w];
+      st_cluster_u64(cluster_map(smem_u32(&s.n[rank]), tid), t);
+    }
+    cluster_sync_all();
+    t = 0;
+    for (int r = 0; r < ctas; ++r) t += s.n[r];
+    total_f = fmaxf((float)t, 1.f);
+  }
+  const bool greedy = p.temperature < 1e-6f;
+  const float inv_t = greedy ? 1.f : 1.0f / p.temperature;
+  // scaled logits into shared memory, their maximum (greedy: and the first place that attains it)
+  float mx = -FLT_MAX;
+  int64_t arg = 0;
+  auto take = [&](int i, float v, uint32_t c) {
+    if (penal && c) { v -= p.presence; v -= p.frequency * ((float)c / total_f); }
+    v *= inv_t;
+    if (v > mx) { mx = v; arg = first + i; }
+    return v;
+  };
+  if (wide) {  // slices and rows are multiples of four at 16-byte addresses
+    const int n4 = n >> 2;
+#pragma unroll 4
+    for (int i = tid; i < n4; i += kRowThreads) {
+      float4 v = reinterpret_cast<const float4*>(x)[i];
+      uint4 c = make_uint4(0, 0, 0, 0);
+      if (penal) c = reinterpret_cast<const uint4*>(cnt)[i];
+      v.x = take(4 * i, v.x, c.x); v.y = take(4 * i + 1, v.y, c.y);
+      v.z = take(4 * i + 2, v.z, c.z); v.w = take(4 * i + 3, v.w, c.w);
+      reinterpret_cast<float4*>(s_q)[i] = v;
+    }
+  } else {
+    for (int i = tid; i < n; i += kRowThreads) s_q[i] = take(i, x[i], penal ? cnt[i] : 0u);
+  }
+  {
+    const float wm = warp_max(mx);
+    if (lane == 0) s.warp_part[warp][0] = wm;
+    __syncthreads();
+  }
+  float own[1] = {warp_max(lane < kRowWarps ? s.warp_part[lane][0] : -FLT_MAX)};
+  const float cta_max = own[0];
+  const float (*all)[2 * kCuts] = exchange(s, turn, own, rank, ctas);
+  float gmax = -FLT_MAX;
+  for (int r = 0; r < ctas; ++r) gmax = fmaxf(gmax, all[r][0]);
+  if (greedy) {
+    // delta distribution on the first maximum (logits_to_probs, mod.rs:79-88)
+    int a = (mx == gmax && cta_max == gmax) ? (int)arg : INT_MAX;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = min(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if (lane == 0) s.warp_arg[warp] = a;
+    __syncthreads();
+    if (tid < ctas) {
+      a = INT_MAX;
+      for (int w = 0; w < kRowWarps; ++w) a = min(a, s.warp_arg[w]);
+      st_cluster_u32(cluster_map(smem_u32(&s.arg[rank]), tid), (uint32_t)a);
+    }
+    cluster_sync_all();
+    int best = INT_MAX;
+    for (int r = 0; r < ctas; ++r) best = min(best, s.arg[r]);
+    for (int i = tid; i < n; i += kRowThreads) pr[i] = first + i == best ? 1.f : 0.f;
+    if (p.tokens && rank == 0 && tid == 0) p.tokens[row] = (uint32_t)best;
+    return;
+  }
+  // softmax.  The slice holds e = exp(logit - maximum) from here on, and the nucleus is sought among
+  // them: a probability is e times one factor, rounded once.  Sums are fp64, a few additions per lane:
+  // what is left of their error would otherwise scale every probability of the row.
+  double sum = 0.0;
+  for (int i = tid; i < n; i += kRowThreads) {
+    const float e = __expf(s_q[i] - gmax);
+    s_q[i] = e;
+    sum += (double)e;
+  }
+  const double total = row_sum(s, 0, sum, rank, ctas);
+  float thr = 0.f;
+  const bool nucleus = p.top_p < 1.0f - 1e-6f;
+  // The maximum itself contributes 1; a sum below one (or none) comes from rows without a finite maximum,
+  // whose probabilities are no numbers.
+  const bool proper = total >= 1.0;
+  const float want = (float)(p.top_p * total);  // mass of the nucleus, in units of e
+  if (nucleus && !proper) thr = FLT_MAX;
+  if (nucleus && proper) {
+    // Nucleus: the tokens with e >= thr, where thr belongs to the token at which the descending cumulative
+    // mass first reaches top_p, i.e. the largest one whose mass from above is still >= top_p.  Sought among
+    // the bit patterns of positive numbers, which are ordered like the numbers: mass(>= lo) >= want >
+    // mass(>= hi), and every pass cuts [lo, hi) in eight, until the tokens in it are few enough for one CTA
+    // to rank.
+    uint32_t hi = __float_as_uint(1.f) + 1u;
+    // all tokens below (1 - top_p) total / V together have no more than 1 - top_p (half of it: rounding)
+    uint32_t lo = __float_as_uint((float)(0.5 * (1.0 - (double)p.top_p) * total / (double)V));
+    if (lo >= hi) lo = 0;
+    float above = 0.f;   // mass(>= hi)
+    bool known = false;  // whether mass(>= lo) >= top_p has been seen
+    int in_band = INT_MAX;
+    while (hi - lo > 1u && in_band > kBandCap) {
+      const uint32_t step = max((hi - lo) >> 3, 1u);
+      float m[2 * kCuts];
+      // cut 0 is lo, the others lie above it
+      uint32_t cut[kCuts];
+#pragma unroll
+      for (int c = 0; c < kCuts; ++c) {
+        cut[c] = min(lo + step * c, hi);
+        m[c] = m[kCuts + c] = 0.f;
+      }
+      for (int i = tid; i < n; i += kRowThreads) {
+        const float q = s_q[i];
+        const uint32_t b = __float_as_uint(q);
+        if (b >= lo && b < hi) {  // (they are not negative)
+#pragma unroll
+          for (int c = 0; c < kCuts; ++c)
+            if (b >= cut[c]) { m[c] += q; m[kCuts + c] += 1.f; }
+        }
+      }
+      cta_sums(s, m);
+      all = exchange(s, turn, m, rank, ctas);
+      uint32_t new_lo = 0, new_hi = hi;
+      float new_above = above, n_hi = 0.f, n_lo = 0.f;
+      bool found = false;
+#pragma unroll
+      for (int c = kCuts - 1; c >= 0; --c) {
+        float mass = above, count = 0.f;
+        for (int r = 0; r < ctas; ++r) { mass += all[r][c]; count += all[r][kCuts + c]; }
+        if (found) continue;
+        if (mass >= want) { found = true; new_lo = cut[c]; n_lo = count; }
+        else { new_hi = cut[c]; new_above = mass; n_hi = count; }
+      }
+      if (!found) {
+        // not even what lies above lo reaches top_p: everything below counts too (or, with lo = 0, rounding
+        // left the whole row short of top_p: all tokens stay)
+        if (lo == 0) { hi = 1u; break; }
+        hi = lo; above = new_above; lo = 0;
+        continue;
+      }
+      known = true;
+      lo = new_lo; hi = new_hi; above = new_above;
+      in_band = (int)(n_lo - n_hi);
+    }
+    thr = __uint_as_float(lo);
+    if (known && hi - lo > 1u) {
+      // the band's probabilities meet in the first CTA
+      const uint32_t n_addr = cluster_map(smem_u32(&s.n_band), 0), band = cluster_map(smem_u32(&s.band[0]), 0);
+      for (int i = tid; i < n; i += kRowThreads) {
+        const float q = s_q[i];
+        const uint32_t b = __float_as_uint(q);
+        if (b >= lo && b < hi) {
+          uint32_t at;
+          asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(n_addr) : "memory");
+          if (at < (uint32_t)kBandCap) st_cluster_f32(band + 4 * at, q);
+        }
+      }
+      cluster_sync_all();
+      if (rank == 0) {
+        // of every one: the mass from above, in units of 2^-36 so that the order of arrival does not matter
+        const int nb = min(s.n_band, kBandCap);
+        auto fixed = [](float q) { return (unsigned long long)((double)q * 68719476736.0); };
+        const unsigned long long least = fixed(want), from = fixed(above);
+        uint32_t best = 0;
+        if (tid < nb) {
+          const float mine = s.band[tid];
+          unsigned long long m = from;
+          for (int j = 0; j < nb; ++j) {
+            const float q = s.band[j];
+            if (q >= mine) m += fixed(q);
+          }
+          if (m >= least) best = __float_as_uint(mine);
+        }
+        best = __reduce_max_sync(0xffffffffu, best);
+        if (lane == 0) s.warp_arg[warp] = (int)best;
+        __syncthreads();
+        best = 0;
+        for (int w = 0; w < kRowWarps; ++w) best = max(best, (uint32_t)s.warp_arg[w]);
+        // (none: rounding; the whole band stays)
+        if (best < lo) best = lo;
+        if (tid < ctas) st_cluster_f32(cluster_map(smem_u32(&s.thr), tid), __uint_as_float(best));
+      }
+      cluster_sync_all();
+      thr = s.thr;
+    }
+  }
+  // kept mass, of every warp's run of the slice and of every CTA
+  const int run = (n + kRowWarps * 32 - 1) / (kRowWarps * 32) * 32, w0 = min(n, warp * run), w1 = min(n, w0 + run);
+  double mass = 0.0;
+  for (int i = w0 + lane; i < w1; i += 32)
+    if (s_q[i] >= thr) mass += (double)s_q[i];
+  const double kept_mass = row_sum(s, 1, mass, rank, ctas);
+  const float inv = kept_mass > 0.0 || !nucleus ? (float)(1.0 / (nucleus ? kept_mass : total)) : 0.f;
+  auto result = [&](float q) { return !nucleus || q >= thr ? q * inv : 0.f; };
+  if (wide) {
+    const int n4 = n >> 2;
+    for (int i = tid; i < n4; i += kRowThreads) {
+      const float4 v = reinterpret_cast<const float4*>(s_q)[i];
+      reinterpret_cast<float4*>(pr)[i] = make_float4(result(v.x), result(v.y), result(v.z), result(v.w));
+    }
+  } else {
+    for (int i = tid; i < n; i += kRowThreads) pr[i] = result(s_q[i]);
+  }
+  if (!p.tokens) return;
+  // draw: first index whose inclusive cumulative probability exceeds u * total, in index order; where
+  // rounding leaves the target at or past the total, the last token with mass
+  const double target = (double)uniform_from_seed(p.seeds[row]) * kept_mass;
+  double before = 0.0;
+  int chosen = -1, last = -1;
+  for (int r = 0; r < ctas; ++r) {
+    const double m = s.total[1][r];
+    if (m > 0.0) last = r;
+    if (chosen < 0) {
+      if (m > 0.0 && before + m > target) chosen = r;
+      else before += m;
+    }
+  }
+  const bool past = chosen < 0;
+  if (past) chosen = last;
+  if (chosen < 0 || !proper) {  // a row without any mass, or whose masses are no numbers
+    if (rank == 0 && tid == 0) p.tokens[row] = 0;
+    return;
+  }
+  if (rank != chosen) return;
+  int cw = -1, lw = 0;
+  for (int w = 0; w < kRowWarps; ++w) {
+    const double m = s.mass[w];
+    if (m > 0.0) lw = w;
+    if (cw < 0) {
+      if (!past && m > 0.0 && before + m > target) cw = w;
+      else before += m;
+    }
+  }
+  if (cw < 0) cw = lw;
+  if (warp != cw) return;
+  int pick = -1, tail = -1;
+  for (int base = w0; base < w1 && pick < 0; base += 32) {
+    const int i = base + lane;
+    const float q = i < w1 && s_q[i] >= thr ? s_q[i] : 0.f;
+    double incl = q;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const unsigned some = __ballot_sync(0xffffffffu, q > 0.f);
+    const unsigned hit = __ballot_sync(0xffffffffu, q > 0.f && before + incl > target);
+    if (some) tail = base + 31 - __clz(some);
+    if (hit && !past) pick = base + __ffs(hit) - 1;
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) p.tokens[row] = (uint32_t)(first + (pick >= 0 ? pick : tail));
+}
+
 static int launch_sample(cudaStream_t st, float* probs, uint32_t* tokens, const float* logits, const uint32_t* counts,
                          const uint64_t* seeds, int64_t n, int64_t vocab, float temperature, float top_p,
                          float presence, float frequency) {
@@ -188,6 +551,38 @@ static int launch_sample(cudaStream_t st, float* probs, uint32_t* tokens, const 
   SampleParams p;
   p.logits = logits; p.counts = counts; p.probs = probs; p.tokens = tokens; p.seeds = seeds;
   p.vocab = vocab; p.temperature = temperature; p.top_p = top_p; p.presence = presence; p.frequency = frequency;
+  // a CTA per 4096 tokens, a power of two of them
+  int ctas = 1;
+  while (ctas < kRowCtas && (int64_t)ctas * 4096 < vocab) ctas *= 2;
+  const int64_t slice = ((vocab + ctas - 1) / ctas + 3) / 4 * 4;
+  if (slice <= kSliceCap && n <= 65535) {
+    int dev = 0;
+    HB_CUDA_CHECK(cudaGetDevice(&dev));
+    {
+      static bool done[64] = {false};
+      static std::mutex mu;
+      std::lock_guard<std::mutex> lock(mu);
+      if (dev >= 0 && dev < 64 && !done[dev]) {
+        HB_CUDA_CHECK(cudaFuncSetAttribute(sample_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSliceCap * 4));
+        done[dev] = true;
+      }
+    }
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    const int wide = vocab % 4 == 0 && al16(logits) && al16(probs) && al16(counts);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas, (unsigned)n);
+    cfg.blockDim = dim3(kRowThreads);
+    cfg.dynamicSmemBytes = (size_t)slice * 4;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, sample_row_kernel, p, (int)slice, wide));
+    return HB_OK;
+  }
   sample_kernel<<<(unsigned)n, kSampleThreads, 0, st>>>(p);
   HB_LAUNCH_CHECK();
   return HB_OK;
