@@ -309,6 +309,42 @@ def test_argmax_first_maximum(hb, cuda):
     assert got.tolist() == np.argmax(x, axis=1).tolist()
 
 
+# Above 128 rows: tiles of 256 rows by 128 to 256 columns.  Edges: one row past a tile, ragged last tiles in both
+# directions, K of less than a chunk and of a partial last one, N that is no multiple of 16 (scalar stores) and the
+# deep K that stays with the other kernel.
+@pytest.mark.parametrize("M,N,K_", [(129, 16, 8), (256, 256, 64), (257, 4096, 1024), (300, 1000, 200), (512, 6144, 4096),
+                                    (1351, 1408, 2048), (200, 37, 72), (140, 2048, 8192), (700, 2048, 8200)])
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+def test_gemm_many_rows(hb, cuda, M, N, K_, dtype):
+    g = torch.Generator().manual_seed(M + N + K_)
+    x = torch.randn(M, K_, generator=g).to(cuda, TORCH[dtype])
+    w = (torch.randn(N, K_, generator=g) * 0.02).to(cuda, TORCH[dtype])
+    want = x.double() @ w.double().T
+    room = (x.double().abs() @ w.double().abs().T) * K_ * 2.0 ** -24 + 2.0 ** -25  # K fp32 additions
+    unit = 2.0 ** (-8 if dtype == "bf16" else -11)  # rounding of the result (8 and 11 bits)
+    y = hb.gemm(x, w)
+    assert bool(((y.double() - want).abs() <= want.abs() * unit + room).all())
+    if dtype == "bf16":
+        y = hb.gemm_ex(x, w, out_f32=True)
+        assert bool(((y.double() - want).abs() <= room).all())
+        again = hb.gemm_ex(x, w, out_f32=True)
+        assert torch.equal(y, again)
+
+
+@pytest.mark.parametrize("M,I,K_", [(129, 8, 64), (300, 1000, 520), (513, 1792, 1024), (1100, 14336, 256)])
+def test_gemm_swiglu_many_rows(hb, cuda, M, I, K_):
+    g = torch.Generator().manual_seed(M + I)
+    x = torch.randn(M, K_, generator=g).to(cuda, torch.bfloat16)
+    w = (torch.randn(2 * I, K_, generator=g) * 0.05).to(cuda, torch.bfloat16)
+    y = hb.gemm_ex(x, w, epilogue=1)
+    gate, up = (x.double() @ w.double().T).split(I, dim=1)
+    want = torch.nn.functional.silu(gate) * up
+    # bf16 rounding; exponential and division within 2^-20; K fp32 additions in both factors (|silu'| < 1.1)
+    room = (x.double().abs() @ w.double().abs().T) * K_ * 2.0 ** -24
+    room = room[:, :I] * 1.1 * up.abs() + room[:, I:] * gate.abs()
+    assert bool(((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -20) + room + 2.0 ** -30).all())
+
+
 @pytest.mark.parametrize("M,I,K_", [(16, 1024, 512), (64, 14336, 4096), (128, 3584, 8192), (128, 7168, 8192),
                                     (5, 688, 256)])
 @pytest.mark.parametrize("splits", [0, 1, 3])

@@ -162,6 +162,8 @@ struct TcGemmPlan {
   bool out_f32 = false;
   hb_dtype dtype = HB_BF16;  // of X, W and 16-bit outputs
   bool tma_store = false;  // output rows are 16-byte multiples: bulk tensor stores
+  bool pair = false;       // kernel for many rows (gemm_pair.cu): tiles of 256 rows x tile_n accumulator columns
+  int tile_n = 0;
   // scratch layout inside the caller's workspace
   size_t ws_partials_bytes = 0;  // fp32 [m_tiles*n_tiles*splits][m_pad][128]
   size_t ws_counters_bytes = 0;  // int32 [m_tiles*n_tiles] (zero between calls)
@@ -185,5 +187,9 @@ bool gemm_tc_rope_epilogue_ok(const TcGemmPlan& plan);
 int gemm_tc_push_row_block(const TcGemmPlan& plan);
 int gemm_tc_run(const TcGemmPlan& plan, cudaStream_t st, void* Y, int64_t ldy, void* workspace,
                 int* err_flag, const TcNormLink* link = nullptr, const int32_t* tile_group = nullptr);
+
+// Plan and launch of the kernel for many rows (gemm_pair.cu); gemm_tc_plan and gemm_tc_run call them.
+int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceInfo& di);
+int gemm_pair_run(const TcGemmPlan& plan, cudaStream_t st, void* Y, int64_t ldy, int* err_flag, const TcNormLink* link);
 
 }  // namespace hb

@@ -1,0 +1,424 @@
+// GEMM of many batch rows (prompt portions, mixed steps) on pairs of SMs:
+//
+//   Y[M,N] = X[M,K] . W[N,K]^T        M above 128
+//
+// Here the tensor cores are the bound, and behind them the way from L2 to the SMs, so the tile is as
+// large as tensor memory allows: the two CTAs of a pair compute 256 batch rows x tile_n features with
+// tcgen05.mma.cta_group::2.  Each CTA loads its own 128 rows of X (operand A, 128 lanes of its tensor
+// memory) and one half of the tile's weight rows (operand B, shared by the pair), so a CTA moves
+// 16 KB + 64 tile_n bytes per 64 channels instead of the 16 KB + 128 m_pad of a CTA alone.  With SwiGLU
+// the first CTA holds the gate rows and the second the up rows: one accumulator row then has gate j in
+// column j and up j in column tile_n / 2 + j.
+//
+// The kernel is persistent: one pair per two SMs walks over the tiles (batch tiles fastest, so that the
+// tiles that meet the same weights run side by side and weights leave HBM once).  Two accumulators of
+// 256 columns fill tensor memory; four warps empty one while the tensor cores fill the other.  A thread
+// of the epilogue owns one batch row, so its outputs are runs of neighbouring features: 16-byte stores,
+// without a detour through shared memory.
+//
+// Measured (us, before: gemm_tc.cu with tiles of 128 rows): 14336 x 4096 at 1500 rows 151 -> 121
+// (1455 TFLOP/s), 28672 x 4096 SwiGLU at 512 rows 105 -> 88 (1366) and at 3000 rows 532 -> 436 (1616),
+// 4096 x 4096 at 512 rows 22.8 -> 16.9 (1014).
+//
+//   warp 0: TMA producer (both CTAs)      warp 1: MMA issuer (first CTA)
+//   warp 2: tensor memory                 warps 4-7: epilogue
+//
+// Barriers: `full` of a stage lives in the first CTA and counts the bytes of both; the commit that frees
+// a stage (`empty`) or completes an accumulator (`acc_full`) arrives in both CTAs; the epilogue warps of
+// both CTAs arrive at `acc_empty` of the first.  Every wait is bounded.
+#include <cuda.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "common.h"
+#include "gemm.h"
+#include "gemm_act.cuh"
+#include "tc_core.cuh"
+
+namespace hb {
+
+namespace {
+constexpr int kPairRows = 256;      // batch rows of a pair
+constexpr int kPairThreads = 256;
+constexpr int kPairStages = 8;      // at most
+constexpr int kAccCols = 256;       // tensor-memory columns of an accumulator
+constexpr uint32_t kPairABytes = 128 * kTileK * 2;
+}  // namespace
+
+struct PairParams {
+  int M, N;                 // N: output features
+  int tile_n, out_n;        // columns of the accumulator; output features of a tile
+  int stages, k_chunks;
+  int m_tiles, tiles;
+  int epilogue, out_f32, wide;   // wide: 16-byte stores
+  int up_row_offset;
+  int64_t ldy;
+  void* Y;
+  GatedAct act;
+  const float *gate_bias, *up_bias;
+  // see TcNormLink
+  const float* rowsq_in;
+  int rowsq_stride, rowsq_tiles;
+  float rs_inv_n, rs_eps;
+  uint32_t* ready_mc;
+  uint32_t* ready_calls;
+  uint32_t* ready_ctas;
+  int* err_flag;
+};
+
+// The load may report to the barrier of the pair's other CTA.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t e, uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t cluster_bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
+      ::"r"(dst), "l"(tm), "r"(x), "r"(y), "r"(cluster_bar), "r"(e)
+      : "memory");
+}
+// D (+)= A * B over both CTAs' shared memory, rows 0-127 in the first CTA's tensor memory, 128-255 in the second's.
+__device__ __forceinline__ void umma_pair(uint32_t e, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(e)
+      : "memory");
+}
+// Arrives at the barrier of this offset in both CTAs once the MMAs issued so far have completed.
+__device__ __forceinline__ void tc_commit_pair(uint32_t e, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(bar), "h"((uint16_t)3), "r"(e)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
+// 16 neighbouring outputs of one row
+template <typename T>
+__device__ __forceinline__ void store_16(const PairParams& p, int64_t m, int n, const float (&v)[16]) {
+  if (p.wide && n + 16 <= p.N) {
+    if (p.out_f32) {
+      float4* y = reinterpret_cast<float4*>((float*)p.Y + m * p.ldy + n);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+      uint4 r[2];
+      T* e = reinterpret_cast<T*>(r);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) e[j] = from_f32<T>(v[j]);
+      uint4* y = reinterpret_cast<uint4*>((T*)p.Y + m * p.ldy + n);
+      y[0] = r[0];
+      y[1] = r[1];
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (n + j < p.N) {
+      if (p.out_f32) ((float*)p.Y)[m * p.ldy + n + j] = v[j];
+      else ((T*)p.Y)[m * p.ldy + n + j] = from_f32<T>(v[j]);
+    }
+  }
+}
+
+template <typename T, bool GENERAL>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const PairParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t s_full[kPairStages];
+  __shared__ __align__(8) uint64_t s_empty[kPairStages];
+  __shared__ __align__(8) uint64_t s_acc_full[2];
+  __shared__ __align__(8) uint64_t s_acc_empty[2];
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_abort;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const bool swiglu = p.epilogue == kEpiSwiGLU;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t half_n = (uint32_t)p.tile_n / 2;
+  const uint32_t b_bytes = half_n * kTileK * 2, stage_bytes = kPairABytes + b_bytes;
+
+  if (tid == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(smem_u32(&s_full[s]), 1);
+      mbar_init(smem_u32(&s_empty[s]), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&s_acc_full[b]), 1);
+      mbar_init(smem_u32(&s_acc_empty[b]), 8);  // four epilogue warps of two CTAs
+    }
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(2 * kAccCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers are initialised and their tensor memory is there
+  tc_fence_after();
+  const uint32_t tmem_base = s_tmem;
+
+  // Producer and issuer run in their whole warp (see elect_one); the stage and its parity are counted, not divided.
+  if (warp == 0) {
+    // -------------------------------------------------------------- TMA producer
+    const uint32_t e = elect_one(), expect = rank == 0 ? e : 0u;
+    const uint32_t full0 = cluster_map(smem_u32(&s_full[0]), 0);  // the first CTA's barriers
+    bool ok = true;
+    auto w_row = [&](int tile) {
+      const int n0 = tile / p.m_tiles * p.out_n;
+      return swiglu ? (rank ? p.up_row_offset : 0) + n0 : n0 + (int)(rank * half_n);
+    };
+    // Weights never depend on the previous kernel: the first stages' are requested before waiting for it.
+    int pre = 0;
+    if (pair < p.tiles) {
+      pre = min(p.stages, p.k_chunks);
+      const int wr = w_row(pair);
+      for (int i = 0; i < pre; ++i) {
+        mbar_expect_tx_if(expect, smem_u32(&s_full[i]), 2 * stage_bytes);
+        tma_load_2d_pair(e, smem_base + i * stage_bytes + kPairABytes, &tm_w, i * kTileK, wr, full0 + i * 8);
+      }
+    }
+    pdl_wait();
+    int s = 0;
+    uint32_t ph = 1;  // parity of `empty` that the stage's next use waits for
+    for (int tile = pair; tile < p.tiles && ok; tile += pairs) {
+      const int wr = w_row(tile), xr = tile % p.m_tiles * kPairRows + (int)rank * 128;
+      for (int k = 0; k < p.k_chunks; ++k) {
+        const uint32_t dst = smem_base + s * stage_bytes, bar = full0 + s * 8;
+        if (pre > 0) {
+          --pre;
+        } else {
+          ok = mbar_wait(smem_u32(&s_empty[s]), ph, &s_abort);
+          if (!ok) break;
+          mbar_expect_tx_if(expect, smem_u32(&s_full[s]), 2 * stage_bytes);
+          tma_load_2d_pair(e, dst + kPairABytes, &tm_w, k * kTileK, wr, bar);
+        }
+        tma_load_2d_pair(e, dst, &tm_x, k * kTileK, xr, bar);
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
+      }
+    }
+    pdl_launch_dependents();
+    if (s_abort && rank == 0) {
+      // let the copies that were issued land before shared memory is given back: a barrier is either
+      // between phases or completes the one that is open
+      for (int i = 0; i < p.stages; ++i)
+        for (uint32_t n = 0; n < kSpinLimit / 16 && !mbar_try(smem_u32(&s_full[i]), 0) && !mbar_try(smem_u32(&s_full[i]), 1); ++n) {
+        }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      // -------------------------------------------------------------- MMA issuer
+      const uint32_t e = elect_one();
+      // as make_idesc, with 256 rows
+      const uint32_t idesc = (make_idesc<T>(p.tile_n) & ~(31u << 24)) | ((uint32_t)(kPairRows >> 4) << 24);
+      const uint64_t a0 = make_smem_desc(smem_base), b0 = make_smem_desc(smem_base + kPairABytes);
+      const uint32_t step = stage_bytes >> 4;  // of a descriptor, from stage to stage
+      const uint32_t acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+      int s = 0, n = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int tile = pair; tile < p.tiles && ok; tile += pairs, ++n) {
+        const int buf = n & 1;
+        ok = mbar_wait(smem_u32(&s_acc_empty[buf]), ((uint32_t)(n >> 1) & 1u) ^ 1u, &s_abort);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t acc = acc0 + buf * kAccCols;
+        for (int k = 0; k < p.k_chunks; ++k) {
+          ok = mbar_wait(smem_u32(&s_full[s]), ph, &s_abort);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t a_desc = a0 + (uint64_t)(s * step), b_desc = b0 + (uint64_t)(s * step);
+#pragma unroll
+          for (int q = 0; q < kTileK / kUmmaK; ++q)
+            umma_pair(e, acc, a_desc + (uint64_t)(q * 2), b_desc + (uint64_t)(q * 2), idesc, (k > 0 || q > 0) ? 1u : 0u);
+          tc_commit_pair(e, smem_u32(&s_empty[s]));
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
+        }
+        if (ok) tc_commit_pair(e, smem_u32(&s_acc_full[buf]));
+      }
+    }
+    __syncwarp();
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ epilogue
+    pdl_wait();
+    const int row = (warp - 4) * 32 + lane;
+    const uint32_t t_lane = tmem_base + ((uint32_t)((warp - 4) * 32) << 16);
+    const uint32_t empty0 = cluster_map(smem_u32(&s_acc_empty[0]), 0);
+    const bool single = GENERAL && p.epilogue == kEpiAct;
+    int n = 0;
+    for (int tile = pair; tile < p.tiles; tile += pairs, ++n) {
+      const int buf = n & 1;
+      const int64_t m = (int64_t)(tile % p.m_tiles) * kPairRows + rank * 128 + row;
+      const int n0 = tile / p.m_tiles * p.out_n;
+      float rs = 1.f;
+      if (p.rowsq_in && m < p.M) {  // deferred norm (see TcNormLink), summed in the order of the other GEMM kernel
+        const float4* rq = reinterpret_cast<const float4*>(p.rowsq_in + m * p.rowsq_stride);
+        float a = 0.f;
+        for (int i = 0; i < (p.rowsq_tiles + 3) >> 2; ++i) {
+          const float4 v = __ldcg(rq + i);
+          a += (v.x + v.y) + (v.z + v.w);
+        }
+        rs = rsqrtf(a * p.rs_inv_n + p.rs_eps);
+      }
+      bool ok = mbar_wait(smem_u32(&s_acc_full[buf]), (uint32_t)(n >> 1) & 1u, &s_abort);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t src = t_lane + buf * kAccCols;
+      for (int c = 0; c < p.out_n; c += 16) {
+        float v[16];
+        tmem_ld16(src + c, v);
+        if (p.rowsq_in) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] *= rs;
+        }
+        if (swiglu) {
+          float u[16];
+          tmem_ld16(src + half_n + c, u);
+          if (p.rowsq_in) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) u[j] *= rs;
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            float g = v[j], w = u[j];
+            if (GENERAL && n0 + c + j < p.N) {
+              if (p.gate_bias) g += __ldg(p.gate_bias + n0 + c + j);
+              if (p.up_bias) w += __ldg(p.up_bias + n0 + c + j);
+            }
+            v[j] = gated_f<GENERAL>(g, w, p.act);
+          }
+        }
+        if (single) single_16(v, p.act);
+        if (m < p.M) store_16<T>(p, m, n0 + c, v);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(empty0 + buf * 8);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (s_abort && tid == 0 && p.err_flag) atomicExch(p.err_flag, HB_ERR_TIMEOUT);
+  if (p.ready_mc && tid == 0) {
+    // as in gemm_tc.cu: the CTA that finishes last tells all ranks
+    __threadfence();
+    if (atomicInc(p.ready_ctas, gridDim.x - 1) == gridDim.x - 1) {
+      __threadfence();
+      atomicAdd(p.ready_calls, 1u);
+      asm volatile("multimem.red.release.sys.global.add.u32 [%0], %1;" ::"l"(p.ready_mc), "r"(1u) : "memory");
+    }
+  }
+  cluster_sync_all();  // the partner's MMAs read this CTA's shared memory, its arrivals land in it
+  if (warp == 2)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * kAccCols) : "memory");
+}
+
+// ------------------------------------------------------------------------ host
+int gemm_tc_encode(CUtensorMap* tm, const void* ptr, hb_dtype dtype, int64_t rows, int64_t cols, int box_rows);
+
+// The tile's width, such that the last round over all pairs is full: a chunk of 64 channels takes 0.24 us at
+// 128 columns and 0.39 us at 256 (4096 x 14336 at 512 and 1024 rows), i.e. goes with 80 + tile_n.
+// Multiples of 32: each CTA of the pair brings half of the columns, in units of 16.
+static int pick_tile_n(int64_t M, int64_t n_rows, bool swiglu, int pairs) {
+  const int64_t m_tiles = (M + kPairRows - 1) / kPairRows;
+  int best = 256;
+  int64_t cost = INT64_MAX;
+  for (int t = 256; t >= 128; t -= 32) {
+    const int out = swiglu ? t / 2 : t;
+    const int64_t tiles = (n_rows + out - 1) / out * m_tiles;
+    const int64_t c = (tiles + pairs - 1) / pairs * (80 + t);
+    if (c < cost) { cost = c; best = t; }
+  }
+  return best;
+}
+
+int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceInfo& di) {
+  TcGemmPlan& pl = *plan;
+  const bool swiglu = pl.epilogue == kEpiSwiGLU;
+  pl.pair = true;
+  pl.tile_n = pick_tile_n(pl.M, pl.N, swiglu, di.sm_count / 2);
+  pl.m_pad = 128;
+  pl.m_tiles = (int)((pl.M + 127) / 128);  // above one: several batch tiles to whoever asks
+  const size_t stage = kPairABytes + (size_t)pl.tile_n / 2 * kTileK * 2;
+  pl.stages = (int)std::min<size_t>(kPairStages, 208 * 1024 / stage);
+  pl.smem_bytes = pl.stages * stage + 1024;
+  {
+    int cur = 0;
+    HB_CUDA_CHECK(cudaGetDevice(&cur));
+    static bool dev_done[64] = {false};
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (cur >= 0 && cur < 64 && !dev_done[cur]) {
+      for (auto* k : {gemm_pair_kernel<__nv_bfloat16, false>, gemm_pair_kernel<__nv_bfloat16, true>, gemm_pair_kernel<__half, false>})
+        HB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
+      dev_done[cur] = true;
+    }
+  }
+  int rc = gemm_tc_encode(&pl.tm_w, W, pl.dtype, swiglu ? 2 * pl.N : pl.N, pl.K, pl.tile_n / 2);
+  if (!rc) rc = gemm_tc_encode(&pl.tm_x, X, pl.dtype, pl.M, pl.K, 128);
+  return rc;
+}
+
+int gemm_pair_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, int* err_flag, const TcNormLink* link) {
+  if (link && (link->resid || link->post_scale || link->rope_cs || link->push_ranks))
+    return fail(HB_ERR_INVALID_ARG, "gemm_tc: plans of many rows take row scales and the completion signal only");
+  PairParams p{};
+  const bool swiglu = pl.epilogue == kEpiSwiGLU;
+  p.M = (int)pl.M; p.N = (int)pl.N;
+  p.tile_n = pl.tile_n;
+  p.out_n = swiglu ? pl.tile_n / 2 : pl.tile_n;
+  p.stages = pl.stages;
+  p.k_chunks = (int)((pl.K + kTileK - 1) / kTileK);
+  p.m_tiles = (int)((pl.M + kPairRows - 1) / kPairRows);
+  p.tiles = (int)((pl.N + p.out_n - 1) / p.out_n) * p.m_tiles;
+  p.epilogue = pl.epilogue;
+  p.out_f32 = pl.out_f32 ? 1 : 0;
+  p.up_row_offset = (int)pl.N;
+  p.ldy = ldy;
+  p.Y = Y;
+  p.wide = (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (size_t)ldy * (pl.out_f32 ? 4 : 2) % 16 == 0;
+  p.act = pl.act;
+  p.gate_bias = pl.gate_bias;
+  p.up_bias = pl.up_bias;
+  p.err_flag = err_flag;
+  if (link && link->rowsq_in) {
+    p.rowsq_in = link->rowsq_in;
+    p.rowsq_tiles = link->rowsq_tiles;
+    p.rowsq_stride = link->rowsq_stride;
+    p.rs_inv_n = 1.0f / link->n;
+    p.rs_eps = link->eps;
+  }
+  if (link && link->ready_mc) {
+    if (!link->ready_calls || !link->ready_ctas)
+      return fail(HB_ERR_INVALID_ARG, "gemm_tc: the completion signal needs its two local counters");
+    p.ready_mc = link->ready_mc;
+    p.ready_calls = link->ready_calls;
+    p.ready_ctas = link->ready_ctas;
+  }
+  DeviceInfo di;
+  int dev = 0;
+  HB_CUDA_CHECK(cudaGetDevice(&dev));
+  int rc = device_info(dev, &di);
+  if (rc) return rc;
+  const bool general = !pl.act.silu() || pl.gate_bias || pl.up_bias || pl.epilogue == kEpiAct;
+  if (pl.dtype == HB_F16 && general) return fail(HB_ERR_INVALID_ARG, "gemm_tc: f16 has plain outputs and SwiGLU only");
+  auto* kernel = pl.dtype == HB_F16 ? gemm_pair_kernel<__half, false>
+                 : general ? gemm_pair_kernel<__nv_bfloat16, true> : gemm_pair_kernel<__nv_bfloat16, false>;
+  HB_CUDA_CHECK(launch_pdl(kernel, dim3(2 * (unsigned)std::min(p.tiles, di.sm_count / 2)), dim3(kPairThreads), pl.smem_bytes, st,
+                           pl.tm_w, pl.tm_x, p));
+  return HB_OK;
+}
+
+}  // namespace hb

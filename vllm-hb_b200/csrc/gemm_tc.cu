@@ -889,6 +889,10 @@ static int encode_map(CUtensorMap* tm, const void* ptr, hb_dtype dtype, int64_t 
   return HB_OK;
 }
 
+int gemm_tc_encode(CUtensorMap* tm, const void* ptr, hb_dtype dtype, int64_t rows, int64_t cols, int box_rows) {
+  return encode_map(tm, ptr, dtype, rows, cols, box_rows);
+}
+
 // Output map: [rows, cols] elements, row stride ld elements, box
 // [box_rows, 128 cols], no swizzle (the kernel stages rows of 128 features densely).
 // heads > 0: that many such tensors `step` elements apart.
@@ -919,6 +923,16 @@ bool gemm_tc_heads_supported(int64_t N, int64_t K, bool out_f32, const TcHeads& 
   return h.heads >= 1 && h.heads <= 65535 && K % 8 == 0 && h.ldx % 8 == 0 && h.x_step % 8 == 0 && h.ldx >= K && h.x_step >= K &&
          (N * elt) % 16 == 0 && (h.ldy * elt) % 16 == 0 && (h.y_step * elt) % 16 == 0 && h.y_step >= N &&
          (int64_t)h.heads * N < (1ll << 30);
+}
+
+// Whether the kernel for many rows (gemm_pair.cu) takes a product.  Above 128 rows it is the faster one
+// (us here / there): 6144 x 4096 at 136 rows 23.4 / 17.2, 4096 x 4096 17.7 / 15.2, 28672 x 4096 SwiGLU 55.4 / 47.1,
+// at 1500 rows 61.7 / 51.5, 60.7 / 38.2, 269.7 / 238.7.  What stays here is a deep K under so few tiles that
+// they leave half of the pairs idle: splitting K wins (4096 x 14336 at 136 rows 35.1 / 52.3, at 512 rows 66.3 / 53.7).
+static bool gemm_pair_wanted(int64_t M, int64_t n_rows, int64_t K, int sm_count) {
+  if (M <= 128) return false;
+  const int64_t tiles = (M + 255) / 256 * ((n_rows + 127) / 128);
+  return K < 8192 || 4 * tiles > sm_count;
 }
 
 static int pick_splits(int units, int k_chunks, int slots) {
@@ -979,6 +993,9 @@ int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int6
   if (epilogue == kEpiSwiGLU && N % 2) return fail(HB_ERR_INVALID_ARG, "gemm_tc: SwiGLU needs even N");
   const int64_t n_rows = epilogue == kEpiSwiGLU ? N / 2 : N;  // output features
   pl.N = n_rows;
+  if (gemm_pair_wanted(M, n_rows, K, di.sm_count) && !groups && !heads && force_splits <= 0 &&
+      (epilogue == kEpiStore || epilogue == kEpiSwiGLU || epilogue == kEpiAct))
+    return gemm_pair_plan(plan, X, W, di);
   // At most 128 batch rows per tile: a 256-row tile doubles the activation traffic per weight
   // byte and the exchange per CTA (measured at M = 256: 8192 x 3584 38.0 -> 24.9 us, 8192 x 4096
   // 40.7 -> 26.7 us with two tiles of 128 rows).
@@ -1174,6 +1191,7 @@ int gemm_tc_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, voi
   if (pl.splits > 1 && !pl.cluster && !workspace)
     return fail(HB_ERR_INVALID_ARG, "gemm_tc: split-K plan needs a workspace of %zu bytes",
                 pl.workspace_bytes());
+  if (pl.pair) return gemm_pair_run(pl, st, Y, ldy, err_flag, link);
   TcParams p{};
 #ifdef HB_TC_TRACE
   static std::atomic<int> launch_no{0};
