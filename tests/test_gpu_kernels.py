@@ -309,6 +309,47 @@ def test_argmax_first_maximum(hb, cuda):
     assert got.tolist() == np.argmax(x, axis=1).tolist()
 
 
+# The tensor-core kernel cuts a range over clusters of 1, 2, 4 or 8 CTAs of 2, 4 or 8 warps, as the numbers of sequences and
+# heads and the length of the block tables suggest; empty and one-token contexts, parts without a block.
+@pytest.mark.parametrize("n_seqs,hq,hkv,longest", [(1, 8, 2, 5), (1, 4, 4, 700), (3, 32, 8, 1100), (20, 32, 8, 2300),
+                                                   (80, 16, 16, 130), (2, 64, 8, 3000), (150, 8, 8, 40)])
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+def test_paged_attention_clusters(hb, cuda, n_seqs, hq, hkv, longest, window, dtype):
+    """Bound: weights rounded to 2^-8 (bf16) or held in 22 bits (f16); fp32 scores of 128 products and their exponentials
+    within 2^-13 of the weights; the result rounded once."""
+    g = torch.Generator().manual_seed(n_seqs + longest)
+    lens = torch.randint(1, longest + 1, (n_seqs,), generator=g)
+    lens[0] = longest
+    if n_seqs > 2:
+        lens[1], lens[2] = 0, 1
+    per = (longest + 15) // 16
+    blocks = n_seqs * per
+    tables = torch.randperm(blocks, generator=g).view(n_seqs, per)
+    q = torch.randn(n_seqs, hq, 128, generator=g).to(cuda, TORCH[dtype])
+    k = torch.randn(blocks, hkv, 16, 128, generator=g).to(cuda, TORCH[dtype])
+    v = torch.randn(blocks, hkv, 16, 128, generator=g).to(cuda, TORCH[dtype])
+    for b in range(n_seqs):  # slots past a context may hold anything
+        n = int(lens[b])
+        if n < per * 16:
+            last = tables[b, n // 16]
+            v[last, :, n % 16:] = float("nan")
+            k[last, :, n % 16:] = float("nan")
+    got = hb.paged_decode_attention(q, k, v, tables.int().to(cuda), lens.int().to(cuda), sliding_window=window).double()
+    unit, weight = (2.0 ** -8, 2.0 ** -8) if dtype == "bf16" else (2.0 ** -11, 2.0 ** -20)
+    for b in range(n_seqs):
+        n = int(lens[b])
+        if n == 0:
+            assert not got[b].any()
+            continue
+        first = max(0, n - window) if window else 0
+        at = tables[b].to(cuda)
+        kb, vb = (c[at].transpose(1, 2).reshape(-1, hkv, 128)[first:n].double().transpose(0, 1) for c in (k, v))
+        p = torch.softmax(q[b].double().view(hkv, hq // hkv, 128) @ kb.transpose(1, 2) * 128 ** -0.5, -1)
+        want, room = (p @ vb).reshape(hq, 128), (p @ vb.abs()).reshape(hq, 128)
+        assert bool(((got[b] - want).abs() <= (weight + 2.0 ** -13) * room + unit * want.abs() + 2.0 ** -24).all()), (b, n)
+
+
 # Above 128 rows: tiles of 256 rows by 128 to 256 columns.  Edges: one row past a tile, ragged last tiles in both
 # directions, K of less than a chunk and of a partial last one, N that is no multiple of 16 (scalar stores) and the
 # deep K that stays with the other kernel.

@@ -61,3 +61,37 @@ def test_scheduler_greedy(hb, cuda, tiny):
     drawn = serve.generate(eng, prompts, 5, temperature=1.0, seed=3)
     assert [len(d) for d in drawn] == [5] * 4 and eng.num_free_blocks() == 12
     eng.close()
+
+
+# bf16 with heads of 128: portions of 33 tokens and more run as tiles of 16 positions, shorter ones in groups of four, and
+# steps above 128 rows carry the residual and the norm in the kernel for many rows.
+@pytest.mark.parametrize("sizes", [(300, 1, 17), (33, 32, 1), (257, 0, 0), (130, 3, 47), (1, 5, 0)], ids=str)
+def test_mixed_step_of_tiles_groups_and_tokens(hb, cuda, sizes):
+    shape = dict(hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=1,
+                 vocab_size=2048, rms_norm_eps=1e-5, rope_theta=500000.0)
+    eng = hb.Engine.create_random(shape, seed=5, std=0.02, norm_ones=False, max_seq_len=512, bf16=True, max_batch=320)
+    cfg = R.LlamaTpConfig(**shape)
+    w = {name: eng.get_tensor(name).reshape(s) for name, s in R.tensor_shapes(cfg).items()}
+    oracle = R.LlamaTpOracle(cfg, w, world_size=1, dtype="bf16")
+    rng = np.random.default_rng(sum(sizes))
+    before = (40, 100, 7)  # tokens that every sequence holds already
+    reqs = [rng.integers(0, 2048, b + n).astype(np.uint32) for b, n in zip(before, sizes)]
+    seqs = [eng.create_kv_cache() for _ in reqs]
+    for s, r, b in zip(seqs, reqs, before):
+        eng.forward_with_cache(r[:b], 0, s)
+    entries, where = [], []
+    for i, n in enumerate(sizes):
+        if n:
+            wanted = sorted({0, n // 2, n - 1})
+            entries.append((seqs[i], reqs[i][before[i]:], wanted))
+            where += [(i, before[i] + p) for p in wanted]
+    nxt, logits = eng.step(entries)
+    for (i, p), row, tok in zip(where, logits, nxt):
+        want = oracle.forward(reqs[i][:p + 1].tolist(), 0, oracle.new_cache())
+        assert np.max(np.abs(row - want)) <= 2e-2 * np.max(np.abs(want)), (i, p)
+        assert tok == np.argmax(row)
+    # what the step wrote serves the next one, and a step that wants no logits computes none
+    nxt, logits = eng.step([(seqs[0], np.array([7], dtype=np.uint32), []), (seqs[1], np.array([9], dtype=np.uint32), [0])])
+    want = oracle.forward(reqs[1].tolist() + [9], 0, oracle.new_cache())
+    assert len(logits) == 1 and np.max(np.abs(logits[0] - want)) <= 2e-2 * np.max(np.abs(want))
+    eng.close()

@@ -15,7 +15,10 @@
 #include <cfloat>
 #include <mutex>
 
+#include <algorithm>
+
 #include "common.h"
+#include "ops.h"
 
 namespace hb {
 
@@ -311,13 +314,12 @@ static int dispatch_nrep(int nrep, cudaStream_t st, T* out, float* po, float* pm
   }
 }
 
-// Tensor-core kernel (attention_mma.cu): bf16, head_dim 128, up to 16 query heads per kv head.
-bool paged_attention_mma_supported(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
-                                   int nrep, int head_dim, int64_t num_blocks, int hkv, hb_dtype dtype);
+// Tensor-core kernel (attention_mma.cu): bf16 and f16, head_dim 128, up to 16 query heads per kv head.
 int paged_attention_mma(cudaStream_t st, void* out, float* part_o, float* part_ml, const void* q,
                         int64_t q_stride, const void* k_cache, const void* v_cache, const int32_t* block_tables,
-                        const int32_t* ctx_lens, int64_t n_seqs, int hq, int hkv, int64_t max_blocks,
-                        int64_t num_blocks, int n_splits, int window, int* err_flag, int fresh, int q_group);
+                        const int32_t* ctx_lens, int64_t n_groups, int hq, int hkv, int64_t max_blocks,
+                        int64_t num_blocks, int n_splits, int window, int* err_flag, int fresh, const int2* groups,
+                        bool clustered, int64_t blocks, hb_dtype dtype);
 
 // Internal entry: q rows may sit inside a wider [q|k|v] projection buffer.  err_flag
 // (device int, may be null) is raised when a bounded wait of the tensor-core kernel ran out.
@@ -325,25 +327,45 @@ int paged_attention(cudaStream_t st, void* out, const void* q, int64_t q_stride,
                     const void* v_cache, const int32_t* block_tables, const int32_t* ctx_lens,
                     int64_t n_seqs, int n_q_heads, int n_kv_heads, int head_dim,
                     int64_t max_blocks_per_seq, int64_t num_blocks, int n_splits, void* workspace,
-                    hb_dtype dtype, int* err_flag, int window, int fresh_tokens, int q_group) {
+                    hb_dtype dtype, int* err_flag, int window, int fresh_tokens, const PagedGroups* groups) {
   if (n_seqs == 0) return HB_OK;
   const int nrep = n_q_heads / n_kv_heads;
   float* po = (float*)workspace;
   float* pml = po ? po + (size_t)n_seqs * n_q_heads * n_splits * head_dim : nullptr;
   static const bool force_simt = [] { const char* e = getenv("HB_ATTN"); return e && e[0] == 's'; }();
-  if (!force_simt && paged_attention_mma_supported(q, q_stride, k_cache, v_cache, nrep, head_dim, num_blocks,
-                                                   n_kv_heads, dtype)) {
-    int rc = paged_attention_mma(st, out, po, pml, q, q_stride, k_cache, v_cache, block_tables, ctx_lens, n_seqs,
-                                 n_q_heads, n_kv_heads, max_blocks_per_seq, num_blocks, n_splits, window, err_flag,
-                                 fresh_tokens, q_group);
+  if (!force_simt && paged_attention_mma_supported(q, q_stride, k_cache, v_cache, nrep, head_dim, num_blocks, n_kv_heads, dtype)) {
+    // Splits that fit a cluster need no workspace: their number is chosen here, whatever the caller asked for
+    // (results differ in rounding only); more of them, for single long contexts, keep the caller's.
+    int splits = n_splits;
+    bool clustered = false;
+    int64_t blocks = max_blocks_per_seq;
+    if (groups) {
+      splits = groups->splits;
+      blocks = groups->blocks;
+      clustered = true;
+    } else if (n_splits <= 8) {
+      DeviceInfo di;
+      int device = 0;
+      HB_CUDA_CHECK(cudaGetDevice(&device));
+      int rc = device_info(device, &di);
+      if (rc) return rc;
+      if (window > 0) blocks = std::min<int64_t>(blocks, window / HB_BLOCK_SIZE + 2);
+      splits = paged_attention_mma_splits(n_seqs * n_kv_heads, blocks, di.sm_count);
+      clustered = true;
+    }
+    int rc = paged_attention_mma(st, out, po, pml, q, q_stride, k_cache, v_cache, block_tables, ctx_lens,
+                                 groups ? groups->n : n_seqs, n_q_heads, n_kv_heads, max_blocks_per_seq, num_blocks, splits,
+                                 window, err_flag, fresh_tokens, groups ? groups->list : nullptr, clustered, blocks, dtype);
     if (rc) return rc;
-    if (n_splits > 1) {
-      attn_merge_kernel<__nv_bfloat16><<<(unsigned)(n_seqs * n_q_heads), 128, 0, st>>>(
-          (__nv_bfloat16*)out, po, pml, n_splits, head_dim);
+    if (splits > 1 && !clustered) {
+      HB_DISPATCH_DTYPE(dtype, T, {
+        attn_merge_kernel<T><<<(unsigned)(n_seqs * n_q_heads), 128, 0, st>>>((T*)out, po, pml, n_splits, head_dim);
+      });
       HB_LAUNCH_CHECK();
     }
     return HB_OK;
   }
+  if (groups && groups->list) return fail(HB_ERR_INVALID_ARG, "paged attention: groups of rows need the tensor-core kernel");
   HB_DISPATCH_DTYPE(dtype, T, {
     if (head_dim == 128)
       return (dispatch_nrep<T, 128>(nrep, st, (T*)out, po, pml, (const T*)q, (const T*)k_cache,
@@ -383,7 +405,7 @@ int hb_paged_decode_attention(void* stream, void* out, const void* q, const void
   HB_CHECK_ARG(max_blocks_per_seq > 0 && num_blocks > 0, "hb_paged_decode_attention: bad block counts");
   return hb::paged_attention((cudaStream_t)stream, out, q, (int64_t)n_q_heads * head_dim, k_cache,
                              v_cache, block_tables, ctx_lens, n_seqs, n_q_heads, n_kv_heads,
-                             head_dim, max_blocks_per_seq, num_blocks, n_splits, workspace, dtype, nullptr, 0, -1, 1);
+                             head_dim, max_blocks_per_seq, num_blocks, n_splits, workspace, dtype, nullptr, 0, -1, nullptr);
 }
 
 int hb_paged_decode_attention_window(void* stream, void* out, const void* q, const void* k_cache,
@@ -404,7 +426,7 @@ int hb_paged_decode_attention_window(void* stream, void* out, const void* q, con
   HB_CHECK_ARG(sliding_window >= 0, "hb_paged_decode_attention_window: negative window");
   return hb::paged_attention((cudaStream_t)stream, out, q, (int64_t)n_q_heads * head_dim, k_cache,
                              v_cache, block_tables, ctx_lens, n_seqs, n_q_heads, n_kv_heads, head_dim,
-                             max_blocks_per_seq, num_blocks, n_splits, workspace, dtype, nullptr, sliding_window, -1, 1);
+                             max_blocks_per_seq, num_blocks, n_splits, workspace, dtype, nullptr, sliding_window, -1, nullptr);
 }
 
 }  // extern "C"
@@ -469,7 +491,7 @@ int hb_paged_decode_attention_static(void* stream, void* out, const void* q, con
   if (rc) return rc;
   return hb::paged_attention((cudaStream_t)stream, out, q, (int64_t)n_q_heads * head_dim, k_cache, v_cache,
                              block_tables, ctx_lens, n_seqs, n_q_heads, n_kv_heads, head_dim,
-                             max_blocks_per_seq, num_blocks, n_splits, scratch, dtype, nullptr, 0, -1, 1);
+                             max_blocks_per_seq, num_blocks, n_splits, scratch, dtype, nullptr, 0, -1, nullptr);
 }
 
 }  // extern "C"

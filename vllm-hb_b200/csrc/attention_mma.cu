@@ -1,7 +1,7 @@
-// Paged GQA decode attention on tensor cores (bf16, head_dim 128, up to 16 query heads
+// Paged GQA decode attention on tensor cores (bf16 or f16, head_dim 128, up to 16 query heads
 // per kv head).  Same contract and pool layout as the CUDA-core kernel in attention.cu
 // (src/engine/arch/llama_tp.rs:264-324): out = softmax(q k^T / sqrt(d)) v over the
-// sequence's block table, partials + log-sum-exp merge when the KV range is split.
+// sequence's block table, log-sum-exp merge when the KV range is split.
 //
 // Decode attention is a stream of K and V rows read once.  With 4-8 query heads per
 // kv head the CUDA-core kernel needs ~750 issued instructions per 8 KB of KV, which is
@@ -20,11 +20,16 @@
 //   At the end the warps merge their (m, l, O) through shared memory.
 //   When the caller bounds the tokens that the preceding kernels write (the engine's
 //   step), the ring is filled with older blocks before griddepcontrol.wait.
-//   Prefill chunks (q_group > 1): the rows of the batch are consecutive positions of ONE
-//   sequence; a CTA then takes q_group of them, the 16 MMA rows holding q_group positions x
-//   n_rep heads, each row with its own causal limit, so that the sequence's K and V are read
-//   once per q_group positions instead of once per position (src/engine/arch/llama_tp.rs:
-//   313-316: the causal mask of a multi-token forward).
+//   Split ranges: up to eight CTAs of one (sequence, kv head) form a thread-block cluster and sum
+//   up through each other's shared memory, without a workspace or a second kernel; so a range is
+//   cut wherever that keeps more SMs busy or evens out sequences of different lengths
+//   (paged_attention_mma_splits).  More splits than eight write partials for a merge kernel.
+//   Groups: a CTA may take several rows that are consecutive positions of one sequence, the 16 MMA
+//   rows holding positions x n_rep heads, each row with its own causal limit, so that the
+//   sequence's K and V are read once per group instead of once per position
+//   (src/engine/arch/llama_tp.rs:313-316: the causal mask of a multi-token forward).
+//   f16: weights enter the second product as two f16 numbers (P 2^14 = hi + lo), which keeps the
+//   22 bits that fp32 weights had on the CUDA cores; bf16 rounds them once.
 //
 // Every wait is bounded: on expiry the CTA raises *err_flag (when given), writes NaN
 // to its outputs, lets outstanding copies land and returns.
@@ -33,6 +38,7 @@
 #include <cuda_bf16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "common.h"
 #include "mma_sync.cuh"
@@ -43,18 +49,20 @@ namespace hb {
 constexpr int kAttnStages = 3;
 constexpr int kAttnStageBytes = 8192;  // K lo | K hi | V lo | V hi, 2 KB each
 constexpr int kAttnHD = 128;
+constexpr int kAttnCluster = 8;        // splits that sum up in a cluster, at most
 // shared memory of a CTA of NW warps (the merge scratch [NW][16][132] floats fits inside)
 constexpr size_t mma_attn_smem(int nw) { return (size_t)nw * kAttnStages * kAttnStageBytes + 1024; }
 
-template <int NW>
+template <int NW, typename T>
 __global__ void __launch_bounds__(NW * 32)
 paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                      __nv_bfloat16* __restrict__ out, float* __restrict__ part_o,
-                      float* __restrict__ part_ml, const __nv_bfloat16* __restrict__ q,
+                      T* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, const T* __restrict__ q,
                       const int32_t* __restrict__ block_tables, const int32_t* __restrict__ ctx_lens, int hq,
                       int hkv, int nrep, int64_t max_blocks, int64_t num_blocks, int n_splits, float scale,
-                      int64_t q_stride, int window, int* err_flag, int fresh, int q_group, int n_rows) {
+                      int64_t q_stride, int window, int* err_flag, int fresh, const int2* __restrict__ groups, int clustered) {
   constexpr int kMmaAttnWarps = NW, kMmaAttnThreads = NW * 32;
+  constexpr bool kPair = std::is_same<T, __half>::value;  // weights as two numbers
+  constexpr float kPairScale = 16384.f;
   // fresh >= 0: at most `fresh` tokens at the end of every sequence were written by the
   // kernels right before this one (the current step's K/V); every earlier block of the pool
   // is final, so its copies may start before those kernels have completed.  The context
@@ -64,11 +72,15 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t s_full[kMmaAttnWarps][kAttnStages];
   __shared__ int s_abort;
+  __shared__ float2 s_ml[NW][16], s_part[16];  // (m, l) of a row: every warp's, the CTA's
+  __shared__ float s_wt[NW][16];               // weights of the warps
+  __shared__ float s_cw[kAttnCluster][16], s_cl[16];  // weights of a cluster's CTAs, sums
 
   const int split = blockIdx.x, kvh = blockIdx.y;
   // the CTA's batch rows: [seq, seq + n_q); row seq + j holds position j of the group
-  const int64_t seq = (int64_t)blockIdx.z * q_group;
-  const int n_q = min(q_group, n_rows - (int)seq);
+  const int2 grp = groups ? groups[blockIdx.z] : make_int2((int)blockIdx.z, 1);
+  const int64_t seq = grp.x;
+  const int n_q = grp.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;  // MMA fragment coordinates
 
@@ -148,8 +160,8 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   // ---- query fragments: rows g and g+8 of the padded 16-head tile, all 8 k-steps
   uint32_t qa[8][4];
   {
-    const __nv_bfloat16* q0 = q + (seq + j_lo) * q_stride + ((int64_t)kvh * nrep + g % nrep) * kAttnHD;
-    const __nv_bfloat16* q1 = q + (seq + j_hi) * q_stride + ((int64_t)kvh * nrep + (g + 8) % nrep) * kAttnHD;
+    const T* q0 = q + (seq + j_lo) * q_stride + ((int64_t)kvh * nrep + g % nrep) * kAttnHD;
+    const T* q1 = q + (seq + j_hi) * q_stride + ((int64_t)kvh * nrep + (g + 8) % nrep) * kAttnHD;
     const bool h0 = row_lo, h1 = row_hi;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
@@ -203,8 +215,8 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             base + (uint32_t)((cidx >> 3) * 2048 + r * 128 + (((cidx & 7) ^ (r & 7)) << 4));
         uint32_t k0, k1, k2, k3;
         ldsm_x4(addr, k0, k1, k2, k3);
-        mma_bf16_16816(sc[nt], qa[2 * q4], k0, k1);
-        mma_bf16_16816(sc[nt], qa[2 * q4 + 1], k2, k3);
+        mma_16816<T>(sc[nt], qa[2 * q4], k0, k1);
+        mma_16816<T>(sc[nt], qa[2 * q4 + 1], k2, k3);
       }
     }
     // ---- online softmax (rows g and g+8), fp32
@@ -237,7 +249,7 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       o[nd][0] *= a0; o[nd][1] *= a0;
       o[nd][2] *= a1; o[nd][3] *= a1;
     }
-    uint32_t pa[4];
+    uint32_t pa[4], pl[4];
     {
       float p[2][4];
 #pragma unroll
@@ -249,10 +261,16 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         l0 += p[nt][0] + p[nt][1];
         l1 += p[nt][2] + p[nt][3];
       }
-      pa[0] = pack_bf16(p[0][0], p[0][1]);
-      pa[1] = pack_bf16(p[0][2], p[0][3]);
-      pa[2] = pack_bf16(p[1][0], p[1][1]);
-      pa[3] = pack_bf16(p[1][2], p[1][3]);
+      if (kPair) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          split_f16(p[i >> 1][(i & 1) * 2] * kPairScale, p[i >> 1][(i & 1) * 2 + 1] * kPairScale, pa[i], pl[i]);
+      } else {
+        pa[0] = pack_bf16(p[0][0], p[0][1]);
+        pa[1] = pack_bf16(p[0][2], p[0][3]);
+        pa[2] = pack_bf16(p[1][0], p[1][1]);
+        pa[3] = pack_bf16(p[1][2], p[1][3]);
+      }
     }
     // ---- O[16 heads x 128] += P V
     {
@@ -265,8 +283,12 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             base + 4096u + (uint32_t)((cidx >> 3) * 2048 + r * 128 + (((cidx & 7) ^ (r & 7)) << 4));
         uint32_t v0, v1, v2, v3;
         ldsm_x4_trans(addr, v0, v1, v2, v3);
-        mma_bf16_16816(o[2 * nd2], pa, v0, v1);
-        mma_bf16_16816(o[2 * nd2 + 1], pa, v2, v3);
+        mma_16816<T>(o[2 * nd2], pa, v0, v1);
+        mma_16816<T>(o[2 * nd2 + 1], pa, v2, v3);
+        if (kPair) {
+          mma_16816<T>(o[2 * nd2], pl, v0, v1);
+          mma_16816<T>(o[2 * nd2 + 1], pl, v2, v3);
+        }
       }
     }
     __syncwarp();  // every lane has read the stage
@@ -286,54 +308,119 @@ paged_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   // CTAs hold 100-200 KB of shared memory each while they wait, which the CTAs of this grid
   // that are not resident yet would otherwise miss (measured 4.386 -> 4.367 ms per 8B decode step).
   pdl_trigger();
-  // ---- merge the four warps: (m, l, O) per head through shared memory
+  // ---- merge the warps: (m, l, O) per row through shared memory, the rows that exist
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
   l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   __syncthreads();  // all rings are idle
   constexpr int kOStride = kAttnHD + 4;
-  float* s_o = reinterpret_cast<float*>(smem_gen);             // [4][16][kOStride]
-  float* s_ml = s_o + kMmaAttnWarps * 16 * kOStride;           // [4][16][2]
+  const int rows = n_q * nrep;                       // MMA row h = (position h / nrep, head h % nrep)
+  float* s_o = reinterpret_cast<float*>(smem_gen);  // [warps][16][kOStride]
 #pragma unroll
   for (int nd = 0; nd < 16; ++nd) {
-    *reinterpret_cast<float2*>(s_o + (warp * 16 + g) * kOStride + nd * 8 + 2 * t) = make_float2(o[nd][0], o[nd][1]);
-    *reinterpret_cast<float2*>(s_o + (warp * 16 + g + 8) * kOStride + nd * 8 + 2 * t) = make_float2(o[nd][2], o[nd][3]);
+    if (g < rows)
+      *reinterpret_cast<float2*>(s_o + (warp * 16 + g) * kOStride + nd * 8 + 2 * t) = make_float2(o[nd][0], o[nd][1]);
+    if (g + 8 < rows)
+      *reinterpret_cast<float2*>(s_o + (warp * 16 + g + 8) * kOStride + nd * 8 + 2 * t) = make_float2(o[nd][2], o[nd][3]);
   }
   if (t == 0) {
-    s_ml[(warp * 16 + g) * 2] = m0;
-    s_ml[(warp * 16 + g) * 2 + 1] = l0;
-    s_ml[(warp * 16 + g + 8) * 2] = m1;
-    s_ml[(warp * 16 + g + 8) * 2 + 1] = l1;
+    s_ml[warp][g] = make_float2(m0, l0);
+    s_ml[warp][g + 8] = make_float2(m1, l1);
   }
   __syncthreads();
   const bool failed = s_abort != 0;
   if (failed && tid == 0 && err_flag) atomicExch(err_flag, HB_ERR_TIMEOUT);
-  for (int idx = tid; idx < n_q * nrep * kAttnHD; idx += kMmaAttnThreads) {
-    const int h = idx / kAttnHD, d = idx % kAttnHD;   // h = MMA row = (position h / nrep, head h % nrep)
-    float M = -INFINITY;
+  constexpr float kUnit = kPair ? 1.f / kPairScale : 1.f;
+  if (tid < 16) {  // a row's weights of the warps, and its sum
+    float M = -INFINITY, l = 0.f;
 #pragma unroll
-    for (int w = 0; w < kMmaAttnWarps; ++w) M = fmaxf(M, s_ml[(w * 16 + h) * 2]);
-    float ov = 0.f, l = 0.f;
+    for (int w = 0; w < kMmaAttnWarps; ++w) M = fmaxf(M, s_ml[w][tid].x);
 #pragma unroll
     for (int w = 0; w < kMmaAttnWarps; ++w) {
-      const float mw = s_ml[(w * 16 + h) * 2];
-      const float wt = (mw == -INFINITY) ? 0.f : __expf(mw - M);
-      ov += wt * s_o[(w * 16 + h) * kOStride + d];
-      l += wt * s_ml[(w * 16 + h) * 2 + 1];
+      const float2 ml = s_ml[w][tid];
+      const float wt = ml.x == -INFINITY ? 0.f : __expf(ml.x - M);
+      l += wt * ml.y;
+      s_wt[w][tid] = wt * kUnit;
     }
-    if (failed) { ov = __int_as_float(0x7fc00000); l = 1.f; }
+    // (a failed CTA: not a number, for its partners too)
+    s_part[tid] = failed ? make_float2(INFINITY, 1.f) : make_float2(M, l);
+  }
+  __syncthreads();
+  const float nan = __int_as_float(0x7fc00000);
+  auto put = [&](int h, int d, float4 v, float l) {
     const int64_t head = (seq + h / nrep) * hq + (int64_t)kvh * nrep + h % nrep;
+    T r[4] = {from_f32<T>(l > 0.f ? v.x / l : l == l ? 0.f : l), from_f32<T>(l > 0.f ? v.y / l : l == l ? 0.f : l),
+              from_f32<T>(l > 0.f ? v.z / l : l == l ? 0.f : l), from_f32<T>(l > 0.f ? v.w / l : l == l ? 0.f : l)};
+    T* dst = out + head * kAttnHD + d;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dst[j] = r[j];
+  };
+  for (int idx = tid; idx < rows * (kAttnHD / 4); idx += kMmaAttnThreads) {
+    const int h = idx / (kAttnHD / 4), d = idx % (kAttnHD / 4) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kMmaAttnWarps; ++w) {
+      const float wt = s_wt[w][h];
+      const float4 x = *reinterpret_cast<const float4*>(s_o + (w * 16 + h) * kOStride + d);
+      v.x += wt * x.x; v.y += wt * x.y; v.z += wt * x.z; v.w += wt * x.w;
+    }
+    if (failed) v = make_float4(nan, nan, nan, nan);
     if (n_splits == 1) {
-      out[head * kAttnHD + d] = __float2bfloat16_rn(l > 0.f ? ov / l : 0.f);
+      put(h, d, v, s_part[h].y);
+    } else if (clustered) {
+      *reinterpret_cast<float4*>(s_o + h * kOStride + d) = v;  // the place of warp 0, read by this thread above
     } else {
-      part_o[(head * n_splits + split) * kAttnHD + d] = ov;
+      const int64_t head = (seq + h / nrep) * hq + (int64_t)kvh * nrep + h % nrep;
+      float* dst = part_o + (head * n_splits + split) * kAttnHD + d;
+      dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
       if (d == 0) {
-        part_ml[(head * n_splits + split) * 2 + 0] = M;
-        part_ml[(head * n_splits + split) * 2 + 1] = l;
+        part_ml[(head * n_splits + split) * 2 + 0] = s_part[h].x;
+        part_ml[(head * n_splits + split) * 2 + 1] = s_part[h].y;
       }
     }
   }
+  if (!clustered) return;
+  // ---- merge the cluster: every CTA sums its share of the outputs over all partners
+  cluster_sync_all();
+  const uint32_t o_addr = smem_u32(s_o), part_addr = smem_u32(&s_part[0]);
+  if (tid < 16) {
+    float2 ml[kAttnCluster];
+    float M = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int c = 0; c < kAttnCluster; ++c) {
+      ml[c] = make_float2(-INFINITY, 0.f);
+      if (c < n_splits) {
+        ml[c].x = ld_cluster_f32(cluster_map(part_addr + tid * 8, c));
+        ml[c].y = ld_cluster_f32(cluster_map(part_addr + tid * 8 + 4, c));
+      }
+      M = fmaxf(M, ml[c].x);
+    }
+#pragma unroll
+    for (int c = 0; c < kAttnCluster; ++c) {
+      const float wt = ml[c].x == -INFINITY ? 0.f : __expf(ml[c].x - M);
+      l += wt * ml[c].y;
+      s_cw[c][tid] = wt;
+    }
+    s_cl[tid] = l;
+  }
+  __syncthreads();
+  for (int idx = split * kMmaAttnThreads + tid; idx < rows * (kAttnHD / 4); idx += n_splits * kMmaAttnThreads) {
+    const int h = idx / (kAttnHD / 4), d = idx % (kAttnHD / 4) * 4;
+    float4 x[kAttnCluster], v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < kAttnCluster; ++c)
+      if (c < n_splits) x[c] = ld_cluster_v4(cluster_map(o_addr + (uint32_t)(h * kOStride + d) * 4, c));
+#pragma unroll
+    for (int c = 0; c < kAttnCluster; ++c) {
+      if (c < n_splits) {
+        const float wt = s_cw[c][h];
+        v.x += wt * x[c].x; v.y += wt * x[c].y; v.z += wt * x[c].z; v.w += wt * x[c].w;
+      }
+    }
+    put(h, d, v, s_cl[h]);
+  }
+  cluster_sync_all();  // nobody leaves while a partner still reads its shared memory
 }
 
 // ------------------------------------------------------------------------ host
@@ -372,7 +459,9 @@ static int encode_pool_map(CUtensorMap* tm, const void* pool, int64_t num_blocks
 
 bool paged_attention_mma_supported(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
                                    int nrep, int head_dim, int64_t num_blocks, int hkv, hb_dtype dtype) {
-  if (dtype != HB_BF16 || head_dim != kAttnHD || nrep < 1 || nrep > 16) return false;
+  if ((dtype != HB_BF16 && dtype != HB_F16) || head_dim != kAttnHD || nrep < 1 || nrep > 16) return false;
+  // (f16: the head counts that the CUDA-core kernel takes too, no more)
+  if (dtype == HB_F16 && (nrep > 8 || (nrep & (nrep - 1)))) return false;
   if ((reinterpret_cast<uintptr_t>(k_cache) & 15) || (reinterpret_cast<uintptr_t>(v_cache) & 15)) return false;
   if ((reinterpret_cast<uintptr_t>(q) & 3) || (q_stride & 1)) return false;
   if (num_blocks * hkv * HB_BLOCK_SIZE >= (1ll << 31)) return false;  // TMA row coordinate is an int
@@ -388,30 +477,48 @@ int paged_attention_mma_prepare() {
   HB_CUDA_CHECK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(mu);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    HB_CUDA_CHECK(cudaFuncSetAttribute(paged_attn_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)mma_attn_smem(4)));
-    HB_CUDA_CHECK(cudaFuncSetAttribute(paged_attn_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)mma_attn_smem(2)));
-    HB_CUDA_CHECK(cudaFuncSetAttribute(paged_attn_mma_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)mma_attn_smem(8)));
+    auto opt_in = [](auto* kernel, int nw) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_attn_smem(nw));
+    };
+    HB_CUDA_CHECK(opt_in(paged_attn_mma_kernel<2, __nv_bfloat16>, 2));
+    HB_CUDA_CHECK(opt_in(paged_attn_mma_kernel<4, __nv_bfloat16>, 4));
+    HB_CUDA_CHECK(opt_in(paged_attn_mma_kernel<8, __nv_bfloat16>, 8));
+    HB_CUDA_CHECK(opt_in(paged_attn_mma_kernel<2, __half>, 2));
+    HB_CUDA_CHECK(opt_in(paged_attn_mma_kernel<4, __half>, 4));
+    HB_CUDA_CHECK(opt_in(paged_attn_mma_kernel<8, __half>, 8));
     done[dev] = true;
   }
   return HB_OK;
 }
 
+// In how many parts the range of a (group, kv head) is read: a power of two, at most a cluster's.
+// `units` of them with about `blocks` KV blocks each.  With fewer CTAs than two per SM parts are added as
+// long as each keeps four blocks; beyond, up to six per SM, as long as each keeps 32: sequences differ in
+// length, and whole ones leave SMs without work while the longest is read.  Measured (us, one part / what
+// this gives): 20 sequences of 9000 tokens x 8 kv heads 204.8 / 154.3 (eight parts; four: 182), 100 of 1000 x 8
+// 88.4 / 81.2, and where it stays with one, 60 x 16 with a window of 1000: 81.3 against 92.3 in two.
+// A step of 8 positions behind 1500 tokens: 1005 -> 864.
+int paged_attention_mma_splits(int64_t units, int64_t blocks, int sm_count) {
+  int c = 1;
+  while (c < kAttnCluster && ((units * c < 2 * (int64_t)sm_count && blocks >= 8 * c) ||
+                              (units * c < 6 * (int64_t)sm_count && blocks >= 64 * c)))
+    c *= 2;
+  return c;
+}
+
 int paged_attention_mma(cudaStream_t st, void* out, float* part_o, float* part_ml, const void* q,
                         int64_t q_stride, const void* k_cache, const void* v_cache, const int32_t* block_tables,
-                        const int32_t* ctx_lens, int64_t n_seqs, int hq, int hkv, int64_t max_blocks,
-                        int64_t num_blocks, int n_splits, int window, int* err_flag, int fresh, int q_group) {
+                        const int32_t* ctx_lens, int64_t n_groups, int hq, int hkv, int64_t max_blocks,
+                        int64_t num_blocks, int n_splits, int window, int* err_flag, int fresh, const int2* groups,
+                        bool clustered, int64_t blocks, hb_dtype dtype) {
   int rc = paged_attention_mma_prepare();
-  const int nrep_ = hq / hkv;
-  if (q_group < 1 || q_group * nrep_ > 16) return fail(HB_ERR_INVALID_ARG, "paged attention: %d positions x %d heads exceed the 16 rows of a tile", q_group, nrep_);
-  const int n_rows = (int)n_seqs;
   if (rc) return rc;
+  if (n_splits < 2) clustered = false;
+  if (clustered && (n_splits > kAttnCluster || (n_splits & (n_splits - 1))))
+    return fail(HB_ERR_INVALID_ARG, "paged attention: clusters of %d", n_splits);
   CUtensorMap tm_k, tm_v;
   if ((rc = encode_pool_map(&tm_k, k_cache, num_blocks, hkv))) return rc;
   if ((rc = encode_pool_map(&tm_v, v_cache, num_blocks, hkv))) return rc;
-  dim3 grid((unsigned)n_splits, (unsigned)hkv, (unsigned)((n_seqs + q_group - 1) / q_group));
   const float scale = 1.0f / sqrtf((float)kAttnHD);
   // Two CTAs of four warps fit an SM, or four of two warps (same bytes in flight).
   // When the grid is larger than one wave of the former, the smaller CTAs keep every
@@ -420,26 +527,43 @@ int paged_attention_mma(cudaStream_t st, void* out, float* part_o, float* part_m
   int device = 0;
   HB_CUDA_CHECK(cudaGetDevice(&device));
   if ((rc = device_info(device, &di))) return rc;
-  const int64_t ctas = (int64_t)n_splits * hkv * ((n_seqs + q_group - 1) / q_group);
+  const int64_t ctas = (int64_t)n_splits * hkv * n_groups;
   // ... and a grid that does not even fill the SMs takes eight warps per CTA: two warps per
-  // scheduler hide each other's MMA and softmax latency (70B TP=8 shape: 17.2 against 21.0 us)
-  const int nw = ctas > 2 * (int64_t)di.sm_count ? 2 : (ctas <= (int64_t)di.sm_count ? 8 : 4);
-  if (nw == 8) {
-    HB_CUDA_CHECK(launch_pdl(paged_attn_mma_kernel<8>, grid, dim3(256), mma_attn_smem(8), st, tm_k, tm_v,
-                             (__nv_bfloat16*)out, part_o, part_ml, (const __nv_bfloat16*)q, block_tables, ctx_lens, hq,
-                             hkv, hq / hkv, max_blocks, num_blocks, n_splits, scale, q_stride, window, err_flag, fresh, q_group, n_rows));
+  // scheduler hide each other's MMA and softmax latency (70B TP=8 shape: 17.2 against 21.0 us),
+  // unless a part is so short that most of them would only be merged
+  const int nw = ctas > 2 * (int64_t)di.sm_count ? 2 : (ctas <= (int64_t)di.sm_count && blocks >= 8 * n_splits ? 8 : 4);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)n_splits, (unsigned)hkv, (unsigned)n_groups);
+  cfg.blockDim = dim3((unsigned)nw * 32);
+  cfg.dynamicSmemBytes = mma_attn_smem(nw);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (pdl_enabled()) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (clustered) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = (unsigned)n_splits;
+    attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  auto launch = [&](auto* kernel, auto* as) -> int {
+    using T = std::remove_pointer_t<decltype(as)>;
+    HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, tm_k, tm_v, (T*)out, part_o, part_ml, (const T*)q, block_tables, ctx_lens, hq,
+                                     hkv, hq / hkv, max_blocks, num_blocks, n_splits, scale, q_stride, window, err_flag, fresh,
+                                     groups, clustered ? 1 : 0));
     return HB_OK;
-  }
-  if (nw == 2) {
-    HB_CUDA_CHECK(launch_pdl(paged_attn_mma_kernel<2>, grid, dim3(64), mma_attn_smem(2), st, tm_k, tm_v,
-                             (__nv_bfloat16*)out, part_o, part_ml, (const __nv_bfloat16*)q, block_tables, ctx_lens, hq,
-                             hkv, hq / hkv, max_blocks, num_blocks, n_splits, scale, q_stride, window, err_flag, fresh, q_group, n_rows));
-  } else {
-    HB_CUDA_CHECK(launch_pdl(paged_attn_mma_kernel<4>, grid, dim3(128), mma_attn_smem(4), st, tm_k, tm_v,
-                             (__nv_bfloat16*)out, part_o, part_ml, (const __nv_bfloat16*)q, block_tables, ctx_lens, hq,
-                             hkv, hq / hkv, max_blocks, num_blocks, n_splits, scale, q_stride, window, err_flag, fresh, q_group, n_rows));
-  }
-  return HB_OK;
+  };
+  auto of_type = [&](auto* as) -> int {
+    using T = std::remove_pointer_t<decltype(as)>;
+    return nw == 8 ? launch(paged_attn_mma_kernel<8, T>, as) : nw == 2 ? launch(paged_attn_mma_kernel<2, T>, as)
+                                                                    : launch(paged_attn_mma_kernel<4, T>, as);
+  };
+  return dtype == HB_F16 ? of_type((__half*)nullptr) : of_type((__nv_bfloat16*)nullptr);
 }
 
 }  // namespace hb

@@ -217,4 +217,20 @@ int to_f32(cudaStream_t st, float* dst, const void* src, hb_dtype dtype, int64_t
   return HB_OK;
 }
 
+// One CTA per row.
+__global__ void gather_rows_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, const int32_t* __restrict__ rows, int64_t vecs) {
+  pdl_trigger();
+  pdl_grid_wait();
+  const uint4* from = src + (int64_t)rows[blockIdx.x] * vecs;
+  uint4* to = dst + (int64_t)blockIdx.x * vecs;
+  for (int64_t i = threadIdx.x; i < vecs; i += blockDim.x) to[i] = from[i];
+}
+
+int gather_rows(cudaStream_t st, void* dst, const void* src, const int32_t* rows, int64_t n, int64_t row_bytes) {
+  if (row_bytes % 16) return fail(HB_ERR_INVALID_ARG, "gather_rows: rows of %lld bytes", (long long)row_bytes);
+  if (n == 0) return HB_OK;
+  HB_CUDA_CHECK(launch_pdl(gather_rows_kernel, dim3((unsigned)n), dim3(256), 0, st, (uint4*)dst, (const uint4*)src, rows, row_bytes / 16));
+  return HB_OK;
+}
+
 }  // namespace hb

@@ -12,6 +12,7 @@
 //   - no allocation and no host round trip inside a step: all buffers are created at
 //     load, the step is captured once per batch size into a CUDA graph and replayed.
 #include "engine.h"
+#include "layered_ops.h"
 
 namespace hb {
 
@@ -254,6 +255,23 @@ static int alloc_weights(hb_engine* e) {
   return HB_OK;
 }
 
+// The prompt portions' attention of layer l (the tables of a tile's sequence stand at its first row).
+static SpanAttention span_args(const hb_engine* e, int64_t l) {
+  SpanAttention a;
+  a.q = e->d_qkv; a.ld_q = e->qkv_rows;
+  a.out = e->d_attn; a.ld_out = e->hq_l * e->hd;
+  a.kc = e->kc[l]; a.vc = e->vc[l];
+  a.tables = (const int32_t*)(e->d_inputs + e->off_tables);
+  a.max_blocks = e->max_blocks_per_seq; a.num_blocks = e->num_blocks;
+  a.pos = (const int32_t*)(e->d_inputs + e->off_pos);
+  a.heads = (int)e->hq_l; a.kv_heads = (int)e->hkv_l;
+  a.dim = a.vdim = (int)e->hd;
+  a.window = (int)e->window;
+  a.scale = 1.0f / sqrtf((float)e->hd);
+  a.err = e->d_err;
+  return a;
+}
+
 static int alloc_runtime(hb_engine* e, const hb_model_config* cfg) {
   int rc;
   e->max_batch = cfg->max_batch > 0 ? cfg->max_batch : 256;
@@ -280,7 +298,10 @@ static int alloc_runtime(hb_engine* e, const hb_model_config* cfg) {
   e->off_pos = align16(e->off_ids + (size_t)B * 4);
   e->off_ctx = align16(e->off_pos + (size_t)B * 4);
   e->off_slots = align16(e->off_ctx + (size_t)B * 4);
-  e->off_tables = align16(e->off_slots + (size_t)B * 8);
+  e->off_groups = align16(e->off_slots + (size_t)B * 8);
+  e->off_tiles = align16(e->off_groups + (size_t)B * sizeof(int2));
+  e->off_want = align16(e->off_tiles + (size_t)B * sizeof(RowRange));
+  e->off_tables = align16(e->off_want + (size_t)B * 4);
   e->inputs_bytes = align16(e->off_tables + (size_t)B * e->max_blocks_per_seq * 4);
   if ((rc = dev_alloc(e, (void**)&e->d_inputs, e->inputs_bytes))) return rc;
   HB_CUDA_CHECK(cudaMallocHost((void**)&e->h_inputs, e->inputs_bytes));
@@ -307,7 +328,14 @@ static int alloc_runtime(hb_engine* e, const hb_model_config* cfg) {
   if ((rc = hb_rope_inv_freq((float)e->theta, (int)e->hd, inv.data()))) return rc;
   if ((rc = dev_alloc(e, (void**)&e->d_inv_freq, inv.size() * 4))) return rc;
   HB_CUDA_CHECK(cudaMemcpy(e->d_inv_freq, inv.data(), inv.size() * 4, cudaMemcpyHostToDevice));
+  if ((rc = dev_alloc(e, &e->d_xw, (size_t)B * e->H * es))) return rc;
   if ((rc = paged_attention_mma_prepare())) return rc;
+  const int nrep = (int)(e->hq_l / e->hkv_l);
+  const char* simt = getenv("HB_ATTN");
+  e->attn_mma = !(simt && simt[0] == 's') && e->L > 0 &&
+                paged_attention_mma_supported(e->d_qkv, e->qkv_rows, e->kc[0], e->vc[0], nrep, (int)e->hd, e->num_blocks,
+                                              (int)e->hkv_l, e->dtype);
+  e->attn_tile = e->attn_mma ? span_attention_tile_positions(span_args(e, 0), e->dtype) : 0;
   e->attn_ws_bytes = hb_attention_workspace_bytes(B, (int)e->hq_l, (int)e->hd, 16);
   if ((rc = dev_alloc(e, &e->d_attn_ws, e->attn_ws_bytes))) return rc;
   return HB_OK;
@@ -325,7 +353,7 @@ int ensure_gemm_workspace(hb_engine* e, size_t ws) {
   e->gemm_ws_bytes = ws;
   // graphs captured with the old scratch are dropped (it stays allocated until the engine goes)
   for (auto& kv : e->plans)
-    if (kv.second.graph) { cudaGraphExecDestroy(kv.second.graph); kv.second.graph = nullptr; }
+    kv.second.drop_graphs();
   if (e->lm)
     for (auto& kv : e->lm->graphs)
       if (kv.second.exec) { cudaGraphExecDestroy(kv.second.exec); kv.second.exec = nullptr; }
@@ -343,33 +371,20 @@ static int pick_attn_splits(const hb_engine* e, int B) {
   return std::max(1, std::min(s, 16));
 }
 
-// Plans (and the captured graph) of a step of B rows; `chunk`: the rows are consecutive
-// positions of one sequence (a prefill chunk), which lets the attention kernel share the K/V
-// stream among them.
-static int ensure_plans(hb_engine* e, int B, bool chunk, StepPlans** out) {
-  const int key = B | (chunk ? 1 << 20 : 0);
-  auto it = e->plans.find(key);
+// Plans (and the captured graphs) of a step of B rows.
+static int ensure_plans(hb_engine* e, int B, StepPlans** out) {
+  auto it = e->plans.find(B);
   const void* window = e->world ? e->world->mc_base : nullptr;
   if (it != e->plans.end()) {
     if (it->second.mm_window == window) { *out = &it->second; return HB_OK; }
-    // the world's multicast window was attached, detached or replaced since: the captured graph
-    // addresses the old one
-    if (it->second.graph) cudaGraphExecDestroy(it->second.graph);
+    // the world's multicast window was attached, detached or replaced since: the captured graphs
+    // address the old one
+    it->second.drop_graphs();
     e->plans.erase(it);
   }
   StepPlans sp;
   sp.mm_window = window;
   sp.attn_splits = pick_attn_splits(e, B);
-  if (chunk && B > 1) {
-    const int nrep = (int)(e->hq_l / e->hkv_l);
-    const bool tc_attn = !getenv("HB_ATTN") &&
-                         paged_attention_mma_supported(e->d_qkv, e->qkv_rows, e->kc[0], e->vc[0], nrep, (int)e->hd,
-                                                       e->num_blocks, (int)e->hkv_l, e->dtype);
-    if (tc_attn && nrep <= 8) {
-      sp.q_group = 16 / nrep;   // 16 MMA rows = q_group positions x nrep heads
-      sp.attn_splits = 1;
-    }
-  }
   size_t ws = 0;
   if (e->use_tc) {
     sp.layer.resize(e->L * 4);
@@ -450,7 +465,7 @@ static int ensure_plans(hb_engine* e, int B, bool chunk, StepPlans** out) {
     const int rc = ensure_gemm_workspace(e, ws);
     if (rc) return rc;
   }
-  auto ins = e->plans.emplace(key, std::move(sp));
+  auto ins = e->plans.emplace(B, std::move(sp));
   *out = &ins.first->second;
   return HB_OK;
 }
@@ -509,8 +524,8 @@ static int reduce_add_norm(hb_engine* e, void* x_out, const void* norm_w, int B,
   return HB_OK;
 }
 
-// Issues every kernel of one decode step on e->stream (captured or direct).
-static int issue_step(hb_engine* e, StepPlans* sp, int B) {
+// Issues every kernel of one step on e->stream (captured or direct).
+static int issue_step(hb_engine* e, StepPlans* sp, int B, const LlamaStep& s) {
   int rc;
   cudaStream_t st = e->stream;
   const uint32_t* d_ids = (const uint32_t*)(e->d_inputs + e->off_ids);
@@ -518,6 +533,11 @@ static int issue_step(hb_engine* e, StepPlans* sp, int B) {
   const int32_t* d_ctx = (const int32_t*)(e->d_inputs + e->off_ctx);
   const int64_t* d_slots = (const int64_t*)(e->d_inputs + e->off_slots);
   const int32_t* d_tables = (const int32_t*)(e->d_inputs + e->off_tables);
+  PagedGroups groups;
+  groups.list = s.listed ? (const int2*)(e->d_inputs + e->off_groups) : nullptr;
+  groups.n = s.n_groups;
+  groups.splits = s.splits;
+  groups.blocks = s.blocks;
   const float eps = (float)e->eps;
   e->last_launches = 0;
 
@@ -587,11 +607,16 @@ static int issue_step(hb_engine* e, StepPlans* sp, int B) {
     }
     // softmax(q k^T / sqrt d) v over the block table          llama_tp.rs:264-324
     prof_mark(e, kCatAttention);
-    if ((rc = paged_attention(st, e->d_attn, e->d_qkv, e->qkv_rows, e->kc[l], e->vc[l], d_tables,
-                              d_ctx, B, (int)e->hq_l, (int)e->hkv_l, (int)e->hd,
-                              e->max_blocks_per_seq, e->num_blocks, sp->attn_splits, e->d_attn_ws,
-                              e->dtype, e->d_err, (int)e->window, attn_fresh, sp->q_group))) return rc;
-    e->last_launches += 1 + (sp->attn_splits > 1 ? 1 : 0);
+    if (s.n_groups) {
+      if ((rc = paged_attention(st, e->d_attn, e->d_qkv, e->qkv_rows, e->kc[l], e->vc[l], d_tables, d_ctx, B, (int)e->hq_l,
+                                (int)e->hkv_l, (int)e->hd, e->max_blocks_per_seq, e->num_blocks, sp->attn_splits, e->d_attn_ws,
+                                e->dtype, e->d_err, (int)e->window, attn_fresh, e->attn_mma ? &groups : nullptr))) return rc;
+      e->last_launches += 1 + (!e->attn_mma && sp->attn_splits > 1 ? 1 : 0);
+    }
+    if (s.n_tiles) {
+      if ((rc = span_attention_tiles(st, span_args(e, l), (const RowRange*)(e->d_inputs + e->off_tiles), s.n_tiles))) return rc;
+      ++e->last_launches;
+    }
     // o_proj partial, sum over ranks, residual, post-attention norm   llama_tp.rs:327,533-552
     prof_mark(e, kCatGemmO);
     if (sp->push) {
@@ -669,12 +694,25 @@ static int issue_step(hb_engine* e, StepPlans* sp, int B) {
     }
   }
   // logits = x . lm_head^T (fp32 out), greedy argmax            llama_tp.rs:352-355, sampling/mod.rs:105-107
-  prof_mark(e, kCatGemmLmHead);
-  if ((rc = run_gemm(e, sp, 0, kLmHead, e->d_logits, e->d_x, e->lm_head, B, e->V, e->H, true,
-                     defer ? &consume : nullptr))) return rc;
-  prof_mark(e, kCatOther);
-  if ((rc = hb_argmax(st, e->d_next, e->d_logits, B, e->V, HB_F32))) return rc;
-  ++e->last_launches;
+  if (s.want > 0) {
+    prof_mark(e, kCatGemmLmHead);
+    int rows = B;
+    if (s.compact) {
+      // a prompt's logits are wanted for its last token, or for none: the head's product (at 32000 x 4096
+      // a tenth of a step of 512 rows) runs on the wanted rows alone
+      rows = s.want;
+      if ((rc = gather_rows(st, e->d_xw, e->d_x, (const int32_t*)(e->d_inputs + e->off_want), rows, e->H * (int64_t)e->es))) return rc;
+      if (e->use_tc) rc = gemm_tc_run(*s.head, st, e->d_logits, e->V, e->d_gemm_ws, e->d_err);
+      else rc = gemm_simt(st, e->d_logits, e->d_xw, e->lm_head, rows, e->V, e->H, e->dtype, true);
+      if (rc) return rc;
+      e->last_launches += 2;
+    } else if ((rc = run_gemm(e, sp, 0, kLmHead, e->d_logits, e->d_x, e->lm_head, B, e->V, e->H, true, defer ? &consume : nullptr))) {
+      return rc;
+    }
+    prof_mark(e, kCatOther);
+    if ((rc = hb_argmax(st, e->d_next, e->d_logits, rows, e->V, HB_F32))) return rc;
+    ++e->last_launches;
+  }
   prof_mark(e, -1);  // closes the last segment
   return HB_OK;
 }
@@ -758,38 +796,104 @@ static int prefill(hb_engine* e, hb_seq* s, const uint32_t* ids, size_t n, float
   return HB_OK;
 }
 
-// Llama family: every batch row has its own position, context length, KV slot and block table.
+// Prompt portions of at least this many tokens run as tiles, which read a sequence's keys once per 64 rows of
+// queries; shorter ones as groups of the paged kernel, whose ranges can be cut over more CTAs.  With every row of a
+// mixture reading its sequence by itself, and a prompt's rows in fours, a step of 40 decoded tokens and three
+// portions of 437 took 8.98 ms and the prefill of 2000 tokens 12.55 ms; now 6.86 and 9.32 ms (the head's product
+// of the wanted rows alone is 0.4 and 0.6 ms of that).
+constexpr int kTileTokens = 33;
+
+// The head's product of `want` gathered rows.
+static int llama_head_plan(hb_engine* e, int want, TcGemmPlan** out) {
+  const int M = std::min(e->max_batch, (want <= 256 ? (want + 15) / 16 * 16 : (want + 127) / 128 * 128));
+  auto it = e->head_plans.find(M);
+  if (it == e->head_plans.end()) {
+    TcGemmPlan p;
+    int rc = gemm_tc_plan(&p, e->d_xw, e->lm_head, M, e->V, e->H, kEpiStore, true, e->device, 0, nullptr, nullptr, e->dtype);
+    if (rc) return rc;
+    if ((rc = ensure_gemm_workspace(e, p.workspace_bytes()))) return rc;
+    it = e->head_plans.emplace(M, p).first;
+  }
+  *out = &it->second;
+  return HB_OK;
+}
+
+// Llama family: every batch row has its own position, context length and KV slot; block tables stand at
+// the rows whose attention reads them.
 static int llama_prepare(hb_engine* e, const StepBatch& batch, StepExec* x) {
   uint32_t* h_ids = (uint32_t*)(e->h_inputs + e->off_ids);
   int32_t* h_pos = (int32_t*)(e->h_inputs + e->off_pos);
   int32_t* h_ctx = (int32_t*)(e->h_inputs + e->off_ctx);
   int64_t* h_slots = (int64_t*)(e->h_inputs + e->off_slots);
+  int2* h_groups = (int2*)(e->h_inputs + e->off_groups);
+  RowRange* h_tiles = (RowRange*)(e->h_inputs + e->off_tiles);
+  int32_t* h_want = (int32_t*)(e->h_inputs + e->off_want);
   int32_t* h_tables = (int32_t*)(e->h_inputs + e->off_tables);
-  for (const StepSeg& g : batch.segs)
+  LlamaStep& s = x->llama;
+  const int group = e->attn_mma ? std::max<int>(1, 16 / (int)(e->hq_l / e->hkv_l)) : 1;
+  int64_t blocks = 0;  // that the groups read
+  for (const StepSeg& g : batch.segs) {
+    const bool tiles = e->attn_tile > 0 && g.n >= kTileTokens;
     for (int i = 0; i < g.n; ++i) {
       const int b = g.row0 + i;
-      const int64_t pos = g.pos0 + i, need = pos / HB_BLOCK_SIZE + 1;
+      const int64_t pos = g.pos0 + i;
       h_ids[b] = g.tokens[i];
       h_pos[b] = (int32_t)pos;
       h_ctx[b] = (int32_t)(pos + 1);
       h_slots[b] = g.blocks[pos / HB_BLOCK_SIZE] * HB_BLOCK_SIZE + pos % HB_BLOCK_SIZE;
-      int32_t* row = h_tables + (size_t)b * e->max_blocks_per_seq;
-      for (int64_t k = 0; k < need; ++k) row[k] = (int32_t)g.blocks[k];
     }
-  // rows that are consecutive positions of ONE sequence may share the attention's K/V stream
-  const bool chunk = batch.segs.size() == 1 && batch.rows > 1;
-  int rc = ensure_plans(e, batch.rows, chunk, &x->plans);
+    const int step = tiles ? e->attn_tile : group;
+    for (int i = 0; i < g.n; i += step) {
+      const int n = std::min(step, g.n - i);
+      const int64_t need = (g.pos0 + (tiles ? g.n : i + n) - 1) / HB_BLOCK_SIZE + 1;
+      if (!tiles || i == 0) {
+        int32_t* row = h_tables + (size_t)(g.row0 + i) * e->max_blocks_per_seq;
+        for (int64_t k = 0; k < need; ++k) row[k] = (int32_t)g.blocks[k];
+      }
+      if (tiles) {
+        h_tiles[s.n_tiles++] = {g.row0, g.row0 + i, n, i / step};
+      } else {
+        h_groups[s.n_groups++] = make_int2(g.row0 + i, n);
+        blocks += e->window > 0 ? std::min<int64_t>(need, e->window / HB_BLOCK_SIZE + 2) : need;
+      }
+    }
+  }
+  s.listed = s.n_groups != batch.rows;
+  int rc = ensure_plans(e, batch.rows, &x->plans);
   if (rc) return rc;
+  if (s.n_groups && e->attn_mma) {
+    DeviceInfo di;
+    if ((rc = device_info(e->device, &di))) return rc;
+    // (in steps of a power of two, so that few captured graphs follow a context that grows)
+    for (s.blocks = 1; s.blocks * s.n_groups < blocks;) s.blocks *= 2;
+    s.splits = paged_attention_mma_splits((int64_t)s.n_groups * e->hkv_l, s.blocks, di.sm_count);
+  }
+  s.want = (int)batch.want.size();
+  // (up to 128 rows are one tile of the head's product, which streams its weights either way)
+  s.compact = s.want > 0 && s.want < batch.rows && (!e->use_tc || batch.rows > 128) && e->H * (int64_t)e->es % 16 == 0;
+  if (s.compact) {
+    std::copy(batch.want.begin(), batch.want.end(), h_want);
+    if (e->use_tc && (rc = llama_head_plan(e, s.want, &s.head))) return rc;
+  }
   x->rows = batch.rows;
-  // only the used prefix of each region matters; one copy of the whole block is simplest
-  x->input_bytes = e->inputs_bytes;
-  x->graph = &x->plans->graph;
-  x->graph_launches = &x->plans->launches;
-  x->logits_compact = false;
+  // what lies behind the tables of the step's rows need not be copied
+  x->input_bytes = e->off_tables + (size_t)batch.rows * e->max_blocks_per_seq * 4;
+  x->logits_compact = s.compact;
+  // Steps of decoded tokens and portions of a single prompt replay from graphs; in other mixtures the
+  // numbers of tiles and groups hardly ever come again.
+  const bool alone = batch.segs.size() == 1, decode = (int)batch.segs.size() == batch.rows;
+  if ((alone || decode) && (s.want <= 1 || s.want == batch.rows)) {
+    const int wanted = s.want == 0 ? 0 : s.want == batch.rows ? 2 : 1;
+    const bool many = s.blocks >= 8 * s.splits;  // (what the kernel's number of warps asks)
+    const int key = s.splits | wanted << 8 | (decode ? 0 : 1) << 12 | (many ? 1 : 0) << 13;
+    StepPlans::Graph& g = x->plans->graphs[key];
+    x->graph = &g.exec;
+    x->graph_launches = &g.launches;
+  }
   return HB_OK;
 }
 
-static int llama_issue(hb_engine* e, const StepExec& x) { return issue_step(e, x.plans, x.rows); }
+static int llama_issue(hb_engine* e, const StepExec& x) { return issue_step(e, x.plans, x.rows, x.llama); }
 
 // One step of any model family: the batch is checked, its inputs are uploaded in one copy, the
 // kernels replay from a graph (or are issued on the stream), the wanted rows come back.
@@ -1077,8 +1181,7 @@ int hb_engine_free(hb_engine* e) {
   if (!e) return HB_OK;
   cudaSetDevice(e->device);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  for (auto& kv : e->plans)
-    if (kv.second.graph) cudaGraphExecDestroy(kv.second.graph);
+  for (auto& kv : e->plans) kv.second.drop_graphs();
   for (void* p : e->allocations) cudaFree(p);
   if (e->h_swap) cudaFreeHost(e->h_swap);
   if (e->h_inputs) cudaFreeHost(e->h_inputs);

@@ -54,16 +54,25 @@ constexpr int kPairCap = 1024;  // block pairs per copy launch
 struct StepPlans {
   std::vector<TcGemmPlan> layer;  // [L * 4]
   TcGemmPlan lm_head;
-  int attn_splits = 1;
-  int q_group = 1;          // prefill chunks: consecutive positions that share an attention CTA
+  int attn_splits = 1;      // of the CUDA-core attention
   bool defer_norm = false;  // add + norm folded into the GEMM epilogues (TcNormLink)
   bool mm = false;          // exchange through the NVLink switch (multicast window of the world)
   const void* mm_window = nullptr;  // the window the plans (and the captured graph) were made for
   bool rope_epi = false;    // RoPE + KV write folded into the q|k|v GEMM epilogue (TcNormLink)
   bool push = false;        // o_proj / down_proj epilogues push their partials to the reducing ranks (kEpiPush)
   PushGeometry geo_o, geo_down;
-  int64_t launches = 0;  // kernels in one step (fixed per batch size)
-  cudaGraphExec_t graph = nullptr;
+  // captured steps: decoded tokens, or a portion of one prompt, by the parts that the attention cuts ranges
+  // into and by whether logits are asked for (llama_prepare)
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    int64_t launches = 0;  // kernels in it
+  };
+  std::map<int, Graph> graphs;
+  void drop_graphs() {
+    for (auto& g : graphs)
+      if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
+    graphs.clear();
+  }
 };
 
 // ---- one step, as every family sees it
@@ -88,6 +97,17 @@ struct StepBatch {
     rows += n;
   }
 };
+// Llama family: how a step's rows meet the attention kernels, and whose logits are computed.
+struct LlamaStep {
+  int n_groups = 0;      // of the paged kernel: rows by themselves, or in groups (listed)
+  bool listed = false;
+  int splits = 1;        // parts of every group's range
+  int64_t blocks = 0;    // of a group, about
+  int n_tiles = 0;       // tiles of prompt portions (span_attention_tiles)
+  int want = 0;          // rows of logits
+  bool compact = false;  // these rows are gathered before the head's product
+  TcGemmPlan* head = nullptr;  // compact
+};
 // What a family's prepare() decided for the step.
 struct StepExec {
   int rows = 0;
@@ -96,6 +116,7 @@ struct StepExec {
   int64_t* graph_launches = nullptr;
   bool logits_compact = false;          // logits row i belongs to want[i] (else to batch row want[i])
   StepPlans* plans = nullptr;           // Llama family
+  LlamaStep llama;
   LayeredStep layered;                  // layered family
 };
 
@@ -162,9 +183,11 @@ struct hb_engine {
   uint8_t* d_inputs = nullptr;  // Llama family: [ids | positions | ctx | pad | slots | tables]
   uint8_t* h_inputs = nullptr;  // pinned mirror
   size_t inputs_bytes = 0;
-  size_t off_ids = 0, off_pos = 0, off_ctx = 0, off_slots = 0, off_tables = 0;
+  size_t off_ids = 0, off_pos = 0, off_ctx = 0, off_slots = 0, off_groups = 0, off_tiles = 0, off_want = 0, off_tables = 0;
+  bool attn_mma = false;  // the tensor-core paged kernel takes this model
+  int attn_tile = 0;      // positions of a tile of a prompt portion (0: no tiles)
   void *d_h = nullptr, *d_x = nullptr, *d_qkv = nullptr, *d_attn = nullptr, *d_gu = nullptr,
-       *d_act = nullptr, *d_proj = nullptr;
+       *d_act = nullptr, *d_proj = nullptr, *d_xw = nullptr;
   float* d_logits = nullptr;
   std::vector<int> last_rows;  // rows of d_logits the last step filled for its caller, in order
   uint32_t* d_next = nullptr;
@@ -185,6 +208,7 @@ struct hb_engine {
   int sample_rows = 0;
   bool use_tc = false, use_graph = true, fused_swiglu = true;
   std::map<int, hb::StepPlans> plans;
+  std::map<int, hb::TcGemmPlan> head_plans;  // Llama family: of gathered rows, by their (padded) number
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = -1.f;
   int64_t last_launches = 0;

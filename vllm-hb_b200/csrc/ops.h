@@ -5,14 +5,22 @@
 
 namespace hb {
 
+// Rows of the tensor-core kernel in groups of consecutive positions of one sequence, which share a CTA
+// and the K/V stream: list[i] = (first row, rows) with rows * (n_q_heads / n_kv_heads) <= 16, the block
+// table being the first row's (list null: every row by itself).  splits: CTAs (a cluster) per group and
+// kv head, as paged_attention_mma_splits gives them for `blocks` KV blocks per group.
+struct PagedGroups {
+  const int2* list = nullptr;
+  int n = 0, splits = 1;
+  int64_t blocks = 0;
+};
+int paged_attention_mma_splits(int64_t units, int64_t blocks, int sm_count);
 int paged_attention(cudaStream_t st, void* out, const void* q, int64_t q_stride, const void* k_cache,
                     const void* v_cache, const int32_t* block_tables, const int32_t* ctx_lens,
                     int64_t n_seqs, int n_q_heads, int n_kv_heads, int head_dim,
                     int64_t max_blocks_per_seq, int64_t num_blocks, int n_splits, void* workspace,
-                    hb_dtype dtype, int* err_flag = nullptr, int window = 0, int fresh_tokens = -1, int q_group = 1);
-// q_group > 1 (tensor-core kernel only): the rows are consecutive positions of ONE sequence
-// with the same block table (a prefill chunk); q_group of them share a CTA and the K/V stream.
-// Must satisfy q_group * (n_q_heads / n_kv_heads) <= 16 and needs n_splits == 1.
+                    hb_dtype dtype, int* err_flag = nullptr, int window = 0, int fresh_tokens = -1,
+                    const PagedGroups* groups = nullptr);
 // fresh_tokens >= 0: at most that many tokens at the end of every sequence were written by the
 // kernels launched right before this one; blocks of older tokens may be fetched before those
 // kernels have completed (programmatic launch).  -1: nothing is fetched early.
@@ -45,6 +53,9 @@ int rope_kv_write(cudaStream_t st, void* qkv, void* k_cache, void* v_cache,
 // as rope_kv_write rounds them (consumed by the GEMM epilogue that rotates q and k).
 int rope_table(cudaStream_t st, float2* table, const int32_t* positions, const float* inv_freq,
                int64_t n_tokens, int head_dim, hb_dtype dtype);
+
+// dst[i] = src[rows[i]], rows of row_bytes (a multiple of 16).
+int gather_rows(cudaStream_t st, void* dst, const void* src, const int32_t* rows, int64_t n, int64_t row_bytes);
 
 // Fill a [rows, cols] slice of a global [g_rows, g_cols] tensor with N(0, std) drawn
 // from a counter-based generator keyed by (seed, tensor id, global element index).
