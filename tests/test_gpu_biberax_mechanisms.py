@@ -425,6 +425,15 @@ def test_mixture_of_experts(hb, cuda, rows, width, experts, top, ff, m_pad, shar
     Experts(hb, rows, width, experts, top, ff, dtype, m_pad, seed=rows, shared_ff=shared_ff).check()
 
 
+# Several tiles of 128 rows per expert: pairs of them run on pairs of SMs; odd counts, an expert without rows (skew), widths that
+# end inside a tile of features or a chunk of channels.
+@pytest.mark.parametrize("rows,width,experts,top,ff,skew", [(700, 256, 4, 2, 136, 0.0), (300, 200, 2, 1, 520, 0.0),
+                                                            (1000, 128, 5, 2, 1000, 2.0), (260, 72, 1, 1, 40, 0.0)])
+def test_mixture_of_experts_with_many_rows_each(hb, cuda, rows, width, experts, top, ff, skew):
+    e = Experts(hb, rows, width, experts, top, ff, "bf16", 128, seed=rows, skew=skew)
+    e.check()
+
+
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
 def test_everybody_chooses_the_same_experts(hb, cuda, dtype):
     """A router bias that overrides everything: two experts get all rows, the others none."""

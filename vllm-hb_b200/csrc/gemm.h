@@ -189,7 +189,8 @@ int gemm_tc_run(const TcGemmPlan& plan, cudaStream_t st, void* Y, int64_t ldy, v
                 int* err_flag, const TcNormLink* link = nullptr, const int32_t* tile_group = nullptr);
 
 // Plan and launch of the kernel for many rows (gemm_pair.cu); gemm_tc_plan and gemm_tc_run call them.
-int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceInfo& di);
-int gemm_pair_run(const TcGemmPlan& plan, cudaStream_t st, void* Y, int64_t ldy, int* err_flag, const TcNormLink* link);
+int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceInfo& di, const TcGroups* groups);
+int gemm_pair_run(const TcGemmPlan& plan, cudaStream_t st, void* Y, int64_t ldy, int* err_flag, const TcNormLink* link,
+                  const int32_t* tile_group);
 
 }  // namespace hb

@@ -44,6 +44,7 @@ constexpr int kPairThreads = 256;
 constexpr int kPairStages = 8;      // at most
 constexpr int kAccCols = 256;       // tensor-memory columns of an accumulator
 constexpr uint32_t kPairABytes = 128 * kTileK * 2;
+constexpr int kPairListTiles = 256; // tiles of 128 sorted rows that a list holds
 }  // namespace
 
 struct PairParams {
@@ -53,6 +54,8 @@ struct PairParams {
   int m_tiles, tiles;
   int epilogue, out_f32, wide;   // wide: 16-byte stores
   int up_row_offset;
+  const int32_t* tile_group;  // TcGroups: group of every 128 rows
+  int max_tiles, group_rows, n_tiles;
   int64_t ldy;
   void* Y;
   GatedAct act;
@@ -126,7 +129,9 @@ __device__ __forceinline__ void store_16(const PairParams& p, int64_t m, int n, 
   }
 }
 
-template <typename T, bool GENERAL>
+// GROUPS: rows sorted by group (TcGroups) in tiles of 128; a pair takes two tiles of one group, or a last single
+// one, whose second CTA computes the same rows again and stores nothing.
+template <typename T, bool GENERAL, bool GROUPS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -136,6 +141,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   __shared__ __align__(8) uint64_t s_acc_empty[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
+  __shared__ int s_group[GROUPS ? kPairListTiles : 1];
+  __shared__ int2 s_list[GROUPS ? kPairListTiles : 1];  // first tile (-1 - tile: a single one), group
+  __shared__ int s_units;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -168,6 +176,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   cluster_sync_all();  // both CTAs' barriers are initialised and their tensor memory is there
   tc_fence_after();
   const uint32_t tmem_base = s_tmem;
+  int m_tiles = p.m_tiles, tiles = p.tiles;
+  if (GROUPS) {
+    // the previous kernels say whose weights a tile of rows meets
+    pdl_wait();
+    for (int i = tid; i < p.max_tiles; i += kPairThreads) s_group[i] = __ldcg(p.tile_group + i);
+    __syncthreads();
+    if (tid == 0) {
+      int n = 0;
+      for (int i = 0; i < p.max_tiles; ++i) {
+        const int g = s_group[i];
+        if (g < 0) continue;
+        const bool two = i + 1 < p.max_tiles && s_group[i + 1] == g;
+        s_list[n++] = make_int2(two ? i : -1 - i, g);
+        if (two) ++i;
+      }
+      s_units = n;
+    }
+    __syncthreads();
+    m_tiles = s_units;
+    tiles = m_tiles * p.n_tiles;
+  }
+  // Tiles of one pair: batch tiles fastest, so that those that meet the same weights run side by side.
+  auto batch_row = [&](int tile) {  // first row of this CTA
+    if (!GROUPS) return tile % m_tiles * kPairRows + (int)rank * 128;
+    const int t = s_list[tile % m_tiles].x;
+    return t < 0 ? (-1 - t) * 128 : (t + (int)rank) * 128;
+  };
 
   // Producer and issuer run in their whole warp (see elect_one); the stage and its parity are counted, not divided.
   if (warp == 0) {
@@ -176,12 +211,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const uint32_t full0 = cluster_map(smem_u32(&s_full[0]), 0);  // the first CTA's barriers
     bool ok = true;
     auto w_row = [&](int tile) {
-      const int n0 = tile / p.m_tiles * p.out_n;
+      const int n0 = tile / m_tiles * p.out_n + (GROUPS ? s_list[tile % m_tiles].y * p.group_rows : 0);
       return swiglu ? (rank ? p.up_row_offset : 0) + n0 : n0 + (int)(rank * half_n);
     };
     // Weights never depend on the previous kernel: the first stages' are requested before waiting for it.
     int pre = 0;
-    if (pair < p.tiles) {
+    if (!GROUPS && pair < tiles) {
       pre = min(p.stages, p.k_chunks);
       const int wr = w_row(pair);
       for (int i = 0; i < pre; ++i) {
@@ -192,8 +227,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     pdl_wait();
     int s = 0;
     uint32_t ph = 1;  // parity of `empty` that the stage's next use waits for
-    for (int tile = pair; tile < p.tiles && ok; tile += pairs) {
-      const int wr = w_row(tile), xr = tile % p.m_tiles * kPairRows + (int)rank * 128;
+    for (int tile = pair; tile < tiles && ok; tile += pairs) {
+      const int wr = w_row(tile), xr = batch_row(tile);
       for (int k = 0; k < p.k_chunks; ++k) {
         const uint32_t dst = smem_base + s * stage_bytes, bar = full0 + s * 8;
         if (pre > 0) {
@@ -228,7 +263,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       int s = 0, n = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int tile = pair; tile < p.tiles && ok; tile += pairs, ++n) {
+      for (int tile = pair; tile < tiles && ok; tile += pairs, ++n) {
         const int buf = n & 1;
         ok = mbar_wait(smem_u32(&s_acc_empty[buf]), ((uint32_t)(n >> 1) & 1u) ^ 1u, &s_abort);
         if (!ok) break;
@@ -257,10 +292,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const uint32_t empty0 = cluster_map(smem_u32(&s_acc_empty[0]), 0);
     const bool single = GENERAL && p.epilogue == kEpiAct;
     int n = 0;
-    for (int tile = pair; tile < p.tiles; tile += pairs, ++n) {
+    for (int tile = pair; tile < tiles; tile += pairs, ++n) {
       const int buf = n & 1;
-      const int64_t m = (int64_t)(tile % p.m_tiles) * kPairRows + rank * 128 + row;
-      const int n0 = tile / p.m_tiles * p.out_n;
+      const int64_t m = (int64_t)batch_row(tile) + row;
+      const int n0 = tile / m_tiles * p.out_n;
+      const bool mine = m < p.M && !(GROUPS && rank && s_list[tile % m_tiles].x < 0);
       float rs = 1.f;
       if (p.rowsq_in && m < p.M) {  // deferred norm (see TcNormLink), summed in the order of the other GEMM kernel
         const float4* rq = reinterpret_cast<const float4*>(p.rowsq_in + m * p.rowsq_stride);
@@ -301,7 +337,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           }
         }
         if (single) single_16(v, p.act);
-        if (m < p.M) store_16<T>(p, m, n0 + c, v);
+        if (mine) store_16<T>(p, m, n0 + c, v);
       }
       tc_fence_before();
       __syncwarp();
@@ -344,13 +380,15 @@ static int pick_tile_n(int64_t M, int64_t n_rows, bool swiglu, int pairs) {
   return best;
 }
 
-int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceInfo& di) {
+int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceInfo& di, const TcGroups* groups) {
   TcGemmPlan& pl = *plan;
   const bool swiglu = pl.epilogue == kEpiSwiGLU;
   pl.pair = true;
-  pl.tile_n = pick_tile_n(pl.M, pl.N, swiglu, di.sm_count / 2);
+  // (grouped: as many pairs of tiles as are likely)
+  const int64_t likely = groups ? (int64_t)std::max(1, (groups->likely_tiles + 1) / 2) * kPairRows : pl.M;
+  pl.tile_n = pick_tile_n(likely, pl.N, swiglu, di.sm_count / 2);
   pl.m_pad = 128;
-  pl.m_tiles = (int)((pl.M + 127) / 128);  // above one: several batch tiles to whoever asks
+  pl.m_tiles = groups ? groups->max_tiles : (int)((pl.M + 127) / 128);  // above one: several batch tiles to whoever asks
   const size_t stage = kPairABytes + (size_t)pl.tile_n / 2 * kTileK * 2;
   pl.stages = (int)std::min<size_t>(kPairStages, 208 * 1024 / stage);
   pl.smem_bytes = pl.stages * stage + 1024;
@@ -361,17 +399,19 @@ int gemm_pair_plan(TcGemmPlan* plan, const void* X, const void* W, const DeviceI
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
     if (cur >= 0 && cur < 64 && !dev_done[cur]) {
-      for (auto* k : {gemm_pair_kernel<__nv_bfloat16, false>, gemm_pair_kernel<__nv_bfloat16, true>, gemm_pair_kernel<__half, false>})
+      for (auto* k : {gemm_pair_kernel<__nv_bfloat16, false, false>, gemm_pair_kernel<__nv_bfloat16, true, false>,
+                      gemm_pair_kernel<__nv_bfloat16, true, true>, gemm_pair_kernel<__half, false, false>})
         HB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
       dev_done[cur] = true;
     }
   }
-  int rc = gemm_tc_encode(&pl.tm_w, W, pl.dtype, swiglu ? 2 * pl.N : pl.N, pl.K, pl.tile_n / 2);
-  if (!rc) rc = gemm_tc_encode(&pl.tm_x, X, pl.dtype, pl.M, pl.K, 128);
+  const int64_t w_rows = (swiglu ? 2 * pl.N : pl.N) * (groups ? groups->groups : 1);
+  int rc = gemm_tc_encode(&pl.tm_w, W, pl.dtype, w_rows, pl.K, pl.tile_n / 2);
+  if (!rc) rc = gemm_tc_encode(&pl.tm_x, X, pl.dtype, pl.M, groups ? pl.ldx : pl.K, 128);
   return rc;
 }
 
-int gemm_pair_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, int* err_flag, const TcNormLink* link) {
+int gemm_pair_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, int* err_flag, const TcNormLink* link, const int32_t* tile_group) {
   if (link && (link->resid || link->post_scale || link->rope_cs || link->push_ranks))
     return fail(HB_ERR_INVALID_ARG, "gemm_tc: plans of many rows take row scales and the completion signal only");
   PairParams p{};
@@ -382,7 +422,14 @@ int gemm_pair_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, i
   p.stages = pl.stages;
   p.k_chunks = (int)((pl.K + kTileK - 1) / kTileK);
   p.m_tiles = (int)((pl.M + kPairRows - 1) / kPairRows);
-  p.tiles = (int)((pl.N + p.out_n - 1) / p.out_n) * p.m_tiles;
+  p.n_tiles = (int)((pl.N + p.out_n - 1) / p.out_n);
+  p.tiles = p.n_tiles * p.m_tiles;
+  if (pl.groups) {
+    p.tile_group = tile_group;
+    p.max_tiles = pl.m_tiles;
+    p.group_rows = pl.group_rows;
+    p.tiles = p.n_tiles * p.max_tiles;  // at most: what there is is counted on the device
+  }
   p.epilogue = pl.epilogue;
   p.out_f32 = pl.out_f32 ? 1 : 0;
   p.up_row_offset = (int)pl.N;
@@ -414,8 +461,9 @@ int gemm_pair_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, i
   if (rc) return rc;
   const bool general = !pl.act.silu() || pl.gate_bias || pl.up_bias || pl.epilogue == kEpiAct;
   if (pl.dtype == HB_F16 && general) return fail(HB_ERR_INVALID_ARG, "gemm_tc: f16 has plain outputs and SwiGLU only");
-  auto* kernel = pl.dtype == HB_F16 ? gemm_pair_kernel<__half, false>
-                 : general ? gemm_pair_kernel<__nv_bfloat16, true> : gemm_pair_kernel<__nv_bfloat16, false>;
+  auto* kernel = pl.dtype == HB_F16 ? gemm_pair_kernel<__half, false, false>
+                 : pl.groups ? gemm_pair_kernel<__nv_bfloat16, true, true>
+                 : general ? gemm_pair_kernel<__nv_bfloat16, true, false> : gemm_pair_kernel<__nv_bfloat16, false, false>;
   HB_CUDA_CHECK(launch_pdl(kernel, dim3(2 * (unsigned)std::min(p.tiles, di.sm_count / 2)), dim3(kPairThreads), pl.smem_bytes, st,
                            pl.tm_w, pl.tm_x, p));
   return HB_OK;

@@ -995,7 +995,7 @@ int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int6
   pl.N = n_rows;
   if (gemm_pair_wanted(M, n_rows, K, di.sm_count) && !groups && !heads && force_splits <= 0 &&
       (epilogue == kEpiStore || epilogue == kEpiSwiGLU || epilogue == kEpiAct))
-    return gemm_pair_plan(plan, X, W, di);
+    return gemm_pair_plan(plan, X, W, di, nullptr);
   // At most 128 batch rows per tile: a 256-row tile doubles the activation traffic per weight
   // byte and the exchange per CTA (measured at M = 256: 8192 x 3584 38.0 -> 24.9 us, 8192 x 4096
   // 40.7 -> 26.7 us with two tiles of 128 rows).
@@ -1014,6 +1014,12 @@ int gemm_tc_plan(TcGemmPlan* plan, const void* X, const void* W, int64_t M, int6
       k_chunks = std::min(k_chunks, (int)((pl.K2 + kTileK - 1) / kTileK));  // what the split of K can count on
     }
   }
+  // Groups of more than 128 rows each fill the tiles of the kernel for many rows: 8 experts of 150 rows on average,
+  // 14336 x 4096 gate and up and back, 489 us in all here and 387 there.  With one tile per group (likely_tiles ==
+  // groups) the second CTA of every pair would repeat the first one's rows; those stay here.
+  if (groups && !groups->shared_w && groups->m_pad == 128 && groups->max_tiles <= 256 && groups->likely_tiles > groups->groups &&
+      force_splits <= 0)
+    return gemm_pair_plan(plan, X, W, di, groups);
   const bool want_cluster = true;  // split-K partners reduce on chip; global scratch only where a cluster cannot form
   const bool tuned = want_cluster && force_splits <= 0;
   if (groups) pl.m_pad = groups->m_pad;
@@ -1191,7 +1197,7 @@ int gemm_tc_run(const TcGemmPlan& pl, cudaStream_t st, void* Y, int64_t ldy, voi
   if (pl.splits > 1 && !pl.cluster && !workspace)
     return fail(HB_ERR_INVALID_ARG, "gemm_tc: split-K plan needs a workspace of %zu bytes",
                 pl.workspace_bytes());
-  if (pl.pair) return gemm_pair_run(pl, st, Y, ldy, err_flag, link);
+  if (pl.pair) return gemm_pair_run(pl, st, Y, ldy, err_flag, link, tile_group);
   TcParams p{};
 #ifdef HB_TC_TRACE
   static std::atomic<int> launch_no{0};
