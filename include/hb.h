@@ -97,6 +97,10 @@ int hb_rope(void* stream, void* q, void* k, const int32_t* positions, const floa
 int hb_rope_cos_sin(void* stream, void* out, const void* x, const void* cos_table,
                     const void* sin_table, int64_t batch_heads, int64_t seq_len, int head_dim,
                     hb_dtype dtype);
+/* The same of q and k, which share the tables, in one launch where their rows are 16-byte vectors. */
+int hb_rope_cos_sin_pair(void* stream, void* out_q, const void* q, int64_t batch_heads_q, void* out_k,
+                         const void* k, int64_t batch_heads_k, const void* cos_table,
+                         const void* sin_table, int64_t seq_len, int head_dim, hb_dtype dtype);
 
 /* buf[head, offset, :] = src[head, :] for every kv head; buf [nkv, max_seq, head_dim],
  * src [nkv, head_dim]; bit-exact copy, in place (the reference clones the whole buffer

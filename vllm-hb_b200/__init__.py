@@ -209,6 +209,7 @@ _SIGS = {
     "hb_rope_inv_freq": (_i, [_f, _i, _vp]),
     "hb_rope": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i, _i]),
     "hb_rope_cos_sin": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i, _i]),
+    "hb_rope_cos_sin_pair": (_i, [_vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _vp, _i64, _i, _i]),
     "hb_kv_assign_contig": (_i, [_vp, _vp, _vp, _i, _i64, _i, _i64, _i]),
     "hb_kv_assign_paged": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i]),
     "hb_attention_workspace_bytes": (_sz, [_i64, _i, _i, _i]),
@@ -352,13 +353,19 @@ def device_count() -> int:
 
 
 # --------------------------------------------------------------------------- dtypes
+_CODES = {"float32": F32, "float16": F16, "bfloat16": BF16}
+_CODE_OF = {}  # by the dtype itself, as far as seen
+
+
 def dtype_code(t) -> int:
     """Map a torch or numpy dtype to hb_dtype."""
-    name = str(t).replace("torch.", "")
-    try:
-        return {"float32": F32, "float16": F16, "bfloat16": BF16}[name]
-    except KeyError:
-        raise HbError(ERR_UNSUPPORTED_DTYPE, f"unsupported dtype {t}") from None
+    code = _CODE_OF.get(t)
+    if code is None:
+        code = _CODES.get(str(t).replace("torch.", ""))
+        if code is None:
+            raise HbError(ERR_UNSUPPORTED_DTYPE, f"unsupported dtype {t}")
+        _CODE_OF[t] = code
+    return code
 
 
 def _ptr(x) -> Optional[int]:
@@ -377,6 +384,10 @@ def _stream(stream=None) -> Optional[int]:
         try:
             import torch
 
+            # (asking whether there is a GPU and building a Stream object to read its handle took a good part of a
+            # call on one token)
+            if hasattr(torch._C, "_cuda_getCurrentRawStream"):
+                return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
             if torch.cuda.is_available():
                 return torch.cuda.current_stream().cuda_stream
         except Exception:
@@ -428,14 +439,17 @@ class kernels:
             """rope::apply (src/kernels/rope.rs:25): q,k [b,h,s,d], cos/sin [s,d/2]."""
             import torch
 
-            outs = []
-            for x in (q, k):
+            b, h, s, d = q.shape
+            out_q, out_k = torch.empty_like(q), torch.empty_like(k)
+            st, code = _stream(stream), dtype_code(q.dtype)
+            if k.shape[2] == s and k.shape[3] == d and k.dtype == q.dtype:
+                check(lib.hb_rope_cos_sin_pair(st, _ptr(out_q), _ptr(q), b * h, _ptr(out_k), _ptr(k), k.shape[0] * k.shape[1],
+                                               _ptr(cos), _ptr(sin), s, d, code))
+                return out_q, out_k
+            for o, x in ((out_q, q), (out_k, k)):
                 b, h, s, d = x.shape
-                o = torch.empty_like(x)
-                check(lib.hb_rope_cos_sin(_stream(stream), _ptr(o), _ptr(x), _ptr(cos), _ptr(sin),
-                                          b * h, s, d, dtype_code(x.dtype)))
-                outs.append(o)
-            return outs[0], outs[1]
+                check(lib.hb_rope_cos_sin(st, _ptr(o), _ptr(x), _ptr(cos), _ptr(sin), b * h, s, d, dtype_code(x.dtype)))
+            return out_q, out_k
 
         @staticmethod
         def apply_positions(q, k, positions, inv_freq, stream=None):
@@ -523,7 +537,7 @@ def gemm(x, w, stream=None):
     y = torch.empty((M, N), dtype=x.dtype, device=x.device)
     code = dtype_code(x.dtype)
     ws_bytes = lib.hb_gemm_workspace_bytes(M, N, K, code)
-    ws = torch.zeros(max(ws_bytes, 16), dtype=torch.uint8, device=x.device)
+    ws = torch.zeros(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
     check(lib.hb_gemm(_stream(stream), _ptr(y), _ptr(x), _ptr(w), M, N, K, code, _ptr(ws)))
     return y
 

@@ -9,7 +9,8 @@
 extern "C" {
 
 size_t hb_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, hb_dtype dtype) {
-  if (dtype != HB_BF16 || !hb::gemm_tc_supported(M, N, K, dtype)) return 0;
+  // (rows of 16-byte multiples leave through bulk stores: their splits meet in clusters, without scratch)
+  if (dtype != HB_BF16 || N % 8 == 0 || !hb::gemm_tc_supported(M, N, K, dtype)) return 0;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   hb::TcGemmPlan plan;

@@ -87,6 +87,60 @@ rope_cos_sin_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __res
   }
 }
 
+// Rows of 16-byte vectors, of q and then of k (rows_k may be 0): a thread rotates one vector pair
+// (d, d + head_dim / 2).  One launch for both: at one token the launches are what it costs.
+template <typename T>
+__global__ void __launch_bounds__(256)
+rope_cos_sin_vec_kernel(T* __restrict__ out_q, const T* __restrict__ q, int64_t rows_q, T* __restrict__ out_k, const T* __restrict__ k,
+                        int64_t rows_k, const T* __restrict__ cos_t, const T* __restrict__ sin_t, int64_t seq_len, int vph) {
+  constexpr int N = Vec16<T>::N;
+  const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x, r = idx / vph;
+  const int v = (int)(idx % vph), half = vph * N;
+  if (r >= rows_q + rows_k) return;
+  const bool is_q = r < rows_q;
+  const int64_t row = is_q ? r : r - rows_q, t = row % seq_len;
+  const T* x = (is_q ? q : k) + row * 2 * half + v * N;
+  T* y = (is_q ? out_q : out_k) + row * 2 * half + v * N;
+  Vec16<T> a, b, cv, sv;
+  a.load(x);
+  b.load(x + half);
+  cv.load(cos_t + t * half + v * N);
+  sv.load(sin_t + t * half + v * N);
+  float x0[N], x1[N], c[N], s[N], o0[N], o1[N];
+  a.unpack(x0);
+  b.unpack(x1);
+  cv.unpack(c);
+  sv.unpack(s);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    o0[j] = x0[j] * c[j] - x1[j] * s[j];
+    o1[j] = x0[j] * s[j] + x1[j] * c[j];
+  }
+  a.pack(o0);
+  b.pack(o1);
+  a.store(y);
+  b.store(y + half);
+}
+
+// Whether every row of `x` and `out` is made of 16-byte vectors.
+static bool rope_vectors(const void* out, const void* x, const void* cos_t, const void* sin_t, int head_dim, hb_dtype dtype) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) |
+                        reinterpret_cast<uintptr_t>(sin_t);
+  return (all & 15) == 0 && (head_dim / 2 * dtype_size(dtype)) % 16 == 0;
+}
+
+static int rope_vec(cudaStream_t st, void* out_q, const void* q, int64_t rows_q, void* out_k, const void* k, int64_t rows_k,
+                    const void* cos_t, const void* sin_t, int64_t seq_len, int head_dim, hb_dtype dtype) {
+  HB_DISPATCH_DTYPE(dtype, T, {
+    const int vph = head_dim / 2 / Vec16<T>::N;
+    const int64_t ctas = ((rows_q + rows_k) * vph + 255) / 256;
+    rope_cos_sin_vec_kernel<T><<<(unsigned)ctas, 256, 0, st>>>((T*)out_q, (const T*)q, rows_q, (T*)out_k, (const T*)k, rows_k,
+                                                               (const T*)cos_t, (const T*)sin_t, seq_len, vph);
+  });
+  HB_LAUNCH_CHECK();
+  return HB_OK;
+}
+
 }  // namespace hb
 
 extern "C" {
@@ -129,6 +183,9 @@ int hb_rope_cos_sin(void* stream, void* out, const void* x, const void* cos_tabl
   HB_CHECK_ARG(batch_heads >= 0 && seq_len > 0 && batch_heads * seq_len < (1ll << 31),
                "hb_rope_cos_sin: bad shape");
   if (batch_heads == 0) return HB_OK;
+  if (hb::dtype_valid(dtype) && hb::rope_vectors(out, x, cos_table, sin_table, head_dim, dtype))
+    return hb::rope_vec((cudaStream_t)stream, out, x, batch_heads * seq_len, nullptr, nullptr, 0, cos_table, sin_table, seq_len,
+                        head_dim, dtype);
   HB_DISPATCH_DTYPE(dtype, T, {
     hb::rope_cos_sin_kernel<T><<<(unsigned)(batch_heads * seq_len), hb::kRopeThreads, 0,
                                  (cudaStream_t)stream>>>((T*)out, (const T*)x, (const T*)cos_table,
@@ -136,6 +193,22 @@ int hb_rope_cos_sin(void* stream, void* out, const void* x, const void* cos_tabl
   });
   HB_LAUNCH_CHECK();
   return HB_OK;
+}
+
+int hb_rope_cos_sin_pair(void* stream, void* out_q, const void* q, int64_t batch_heads_q, void* out_k, const void* k,
+                         int64_t batch_heads_k, const void* cos_table, const void* sin_table, int64_t seq_len, int head_dim,
+                         hb_dtype dtype) {
+  HB_CHECK_ARG(out_q && q && out_k && k && cos_table && sin_table, "hb_rope_cos_sin_pair: null pointer");
+  HB_CHECK_ARG(head_dim > 0 && head_dim % 2 == 0, "hb_rope_cos_sin_pair: head_dim must be even");
+  HB_CHECK_ARG(batch_heads_q >= 0 && batch_heads_k >= 0 && seq_len > 0 && batch_heads_q * seq_len < (1ll << 31) &&
+                   batch_heads_k * seq_len < (1ll << 31), "hb_rope_cos_sin_pair: bad shape");
+  if (batch_heads_q && batch_heads_k && hb::dtype_valid(dtype) &&
+      hb::rope_vectors(out_q, q, cos_table, sin_table, head_dim, dtype) &&
+      hb::rope_vectors(out_k, k, cos_table, sin_table, head_dim, dtype))
+    return hb::rope_vec((cudaStream_t)stream, out_q, q, batch_heads_q * seq_len, out_k, k, batch_heads_k * seq_len, cos_table,
+                        sin_table, seq_len, head_dim, dtype);
+  const int rc = hb_rope_cos_sin(stream, out_q, q, cos_table, sin_table, batch_heads_q, seq_len, head_dim, dtype);
+  return rc ? rc : hb_rope_cos_sin(stream, out_k, k, cos_table, sin_table, batch_heads_k, seq_len, head_dim, dtype);
 }
 
 }  // extern "C"
