@@ -126,7 +126,8 @@ int hb_kv_assign_paged(void* stream, void* k_cache, void* v_cache, const void* k
  * outside [0, num_blocks) read block 0: nothing outside the tables and the pool is touched).  Query head j reads kv head j / (n_q_heads/n_kv_heads)
  * (src/engine/arch/llama_tp.rs:264-279); scores = q.k/sqrt(d), softmax and the
  * weighted sum accumulate in fp32 (src/engine/arch/llama_tp.rs:304-324).
- * `workspace` holds split-KV partials: hb_attention_workspace_bytes() bytes.
+ * `workspace` holds split-KV partials: hb_attention_workspace_bytes() bytes.  (bf16 and f16 with head_dim 128 choose
+ * the number of parts by themselves up to n_splits = 8, and leave the workspace alone.)
  * Replaces the doc-only stubs of src/attention/ (sdpa.rs:1-11, flash.rs:27-31). */
 size_t hb_attention_workspace_bytes(int64_t n_seqs, int n_q_heads, int head_dim, int n_splits);
 int hb_paged_decode_attention(void* stream, void* out, const void* q, const void* k_cache,
@@ -176,9 +177,9 @@ int hb_paged_decode_attention_static(void* stream, void* out, const void* q, con
 
 /* Y[M,N] = X[M,K] . W[N,K]^T  (weights stored [out,in] and applied as x.W^T, as every
  * matmul of the path does: src/engine/arch/llama_tp.rs:232-234,327,335-337,354).
- * bf16 with K%8==0 runs on tcgen05 tensor cores (swap-AB: the weight's
- * output dim fills the 128-row UMMA M, the batch is the UMMA N; split-K fills the
- * SMs); other dtypes/shapes run a SIMT kernel.  `workspace` (may be NULL when
+ * bf16 with K%8==0, and f16 with K%8==0, N%8==0 and 16-byte addresses, run on tcgen05 tensor cores (up to 128
+ * rows swap-AB: the weight's output dim fills the 128-row UMMA M, the batch is the UMMA N; split-K fills the
+ * SMs; more rows in tiles of 256 on pairs of SMs); other dtypes/shapes run a SIMT kernel.  `workspace` (may be NULL when
  * hb_gemm_workspace_bytes()==0) holds split-K partials and tile counters; it must be
  * zero-initialised once and is left zeroed by every call. */
 size_t hb_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, hb_dtype dtype);
