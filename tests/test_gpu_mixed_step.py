@@ -95,26 +95,3 @@ def test_mixed_step_of_tiles_groups_and_tokens(hb, cuda, sizes):
     want = oracle.forward(reqs[1].tolist() + [9], 0, oracle.new_cache())
     assert len(logits) == 1 and np.max(np.abs(logits[0] - want)) <= 2e-2 * np.max(np.abs(want))
     eng.close()
-
-
-# Tiles of 128 rows hold 128, 32 or 16 positions; portions end inside a tile, contexts inside a step of 64 keys, windows inside
-# a block.  The same prompt in portions of 32 runs through the paged kernel.
-@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (4, 1), (8, 1)])
-@pytest.mark.parametrize("n", [33, 64, 200, 385])
-@pytest.mark.parametrize("window", [0, 70])
-@pytest.mark.parametrize("bf16", [True, False])
-def test_prompt_tiles_against_groups(hb, cuda, heads, kv_heads, n, window, bf16):
-    """Both kernels round each weight (bf16: the paged one to 2^-8) and each output once; two layers of that and of the
-    residual's rounding lie well below 2e-2 of the largest logit, in f16 an eighth of it."""
-    shape = dict(hidden_size=128 * heads, intermediate_size=512, num_hidden_layers=2, num_attention_heads=heads,
-                 num_key_value_heads=kv_heads, vocab_size=1024, rms_norm_eps=1e-5, rope_theta=10000.0, sliding_window=window)
-    ids = np.random.default_rng(n).integers(0, 1024, n + 50).astype(np.uint32)
-    got = []
-    for rows in (512, 32):
-        eng = hb.Engine.create_random(shape, seed=3, std=0.05, max_seq_len=512, bf16=bf16, max_batch=rows)
-        seq = eng.create_kv_cache()
-        first = eng.forward_with_cache(ids[:n], 0, seq)
-        got.append((first, eng.forward_all_positions(ids[n:], n, seq)))  # 50 more: a portion behind a context
-        eng.close()
-    for a, b in zip(*got):
-        assert np.max(np.abs(a - b)) <= (2e-2 if bf16 else 2.5e-3) * np.max(np.abs(b))

@@ -443,7 +443,7 @@ static AttnEncodeFn attn_encode_fn() {
 
 // The pool of one layer as a 2-D tensor [num_blocks * n_kv_heads * 16 rows, 128], box
 // [16 rows, 64 columns], 128-byte swizzle.
-int encode_pool_map(CUtensorMap* tm, const void* pool, int64_t num_blocks, int hkv) {
+static int encode_pool_map(CUtensorMap* tm, const void* pool, int64_t num_blocks, int hkv) {
   AttnEncodeFn enc = attn_encode_fn();
   if (!enc) return fail(HB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   cuuint64_t dims[2] = {(cuuint64_t)kAttnHD, (cuuint64_t)(num_blocks * hkv * HB_BLOCK_SIZE)};

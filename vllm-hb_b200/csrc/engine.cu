@@ -335,8 +335,7 @@ static int alloc_runtime(hb_engine* e, const hb_model_config* cfg) {
   e->attn_mma = !(simt && simt[0] == 's') && e->L > 0 &&
                 paged_attention_mma_supported(e->d_qkv, e->qkv_rows, e->kc[0], e->vc[0], nrep, (int)e->hd, e->num_blocks,
                                               (int)e->hkv_l, e->dtype);
-  e->attn_tile = e->attn_mma ? prompt_attention_positions(span_args(e, 0), e->dtype) : 0;
-  if (e->attn_tile && (rc = prompt_attention_prepare())) return rc;
+  e->attn_tile = e->attn_mma ? span_attention_tile_positions(span_args(e, 0), e->dtype) : 0;
   e->attn_ws_bytes = hb_attention_workspace_bytes(B, (int)e->hq_l, (int)e->hd, 16);
   if ((rc = dev_alloc(e, &e->d_attn_ws, e->attn_ws_bytes))) return rc;
   return HB_OK;
@@ -615,7 +614,7 @@ static int issue_step(hb_engine* e, StepPlans* sp, int B, const LlamaStep& s) {
       e->last_launches += 1 + (!e->attn_mma && sp->attn_splits > 1 ? 1 : 0);
     }
     if (s.n_tiles) {
-      if ((rc = prompt_attention(st, span_args(e, l), (const RowRange*)(e->d_inputs + e->off_tiles), s.n_tiles, e->dtype))) return rc;
+      if ((rc = span_attention_tiles(st, span_args(e, l), (const RowRange*)(e->d_inputs + e->off_tiles), s.n_tiles))) return rc;
       ++e->last_launches;
     }
     // o_proj partial, sum over ranks, residual, post-attention norm   llama_tp.rs:327,533-552
@@ -797,10 +796,10 @@ static int prefill(hb_engine* e, hb_seq* s, const uint32_t* ids, size_t n, float
   return HB_OK;
 }
 
-// Prompt portions of at least this many tokens run as tiles, which read a sequence's keys once per 128 rows of
+// Prompt portions of at least this many tokens run as tiles, which read a sequence's keys once per 64 rows of
 // queries; shorter ones as groups of the paged kernel, whose ranges can be cut over more CTAs.  With every row of a
 // mixture reading its sequence by itself, and a prompt's rows in fours, a step of 40 decoded tokens and three
-// portions of 437 took 8.98 ms and the prefill of 2000 tokens 12.55 ms; now 6.52 and 8.40 ms (the head's product
+// portions of 437 took 8.98 ms and the prefill of 2000 tokens 12.55 ms; now 6.86 and 9.32 ms (the head's product
 // of the wanted rows alone is 0.4 and 0.6 ms of that).
 constexpr int kTileTokens = 33;
 

@@ -103,7 +103,7 @@ struct LlamaStep {
   bool listed = false;
   int splits = 1;        // parts of every group's range
   int64_t blocks = 0;    // of a group, about
-  int n_tiles = 0;       // tiles of prompt portions (prompt_attention)
+  int n_tiles = 0;       // tiles of prompt portions (span_attention_tiles)
   int want = 0;          // rows of logits
   bool compact = false;  // these rows are gathered before the head's product
   TcGemmPlan* head = nullptr;  // compact

@@ -198,12 +198,6 @@ int span_attention_tokens_slots(const SpanAttention& a);
 bool span_attention_tokens_supported(const SpanAttention& a, hb_dtype dtype);
 int span_attention_tiles(cudaStream_t st, const SpanAttention& a, const RowRange* tiles, int n_tiles);
 int span_attention_tokens(cudaStream_t st, const SpanAttention& a, const int32_t* rows, int n_rows, int n_splits, float* part);
-// Prompt portions on tcgen05 (attention_prompt.cu): tiles of up to prompt_attention_positions() consecutive positions
-// (0: these sizes are not taken), with the first row's block table at tables + seg * max_blocks.  prepare: opts in to
-// shared memory, outside any capture.
-int prompt_attention_positions(const SpanAttention& a, hb_dtype dtype);
-int prompt_attention_prepare();
-int prompt_attention(cudaStream_t st, const SpanAttention& a, const RowRange* tiles, int n_tiles, hb_dtype dtype);
 // Whether sizes and alignments suit the tensor-core kernels; the sum of a row's split partials.
 bool span_attention_mma_ok(const SpanAttention& a, hb_dtype dtype);
 int span_attention_merge(cudaStream_t st, const SpanAttention& a, const int32_t* rows, int n_rows, int n_splits, const float* part);
